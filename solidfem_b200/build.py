@@ -24,9 +24,12 @@ CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_COMMON = ["-O3", "-std=c++17", "-lineinfo", "-ccbin", CXX, "-Xcompiler", "-fPIC,-ffp-contract=off",
-               "--expt-relaxed-constexpr"] + ARCH
+               "--expt-relaxed-constexpr", "--split-compile=4"] + ARCH
 CU_SOURCES = {
     "solve.cu": [],
+    "cycle_single.cu": [],
+    "cycle_mixed_storage.cu": [],
+    "cycle_double.cu": [],
     "assembly.cu": ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"],
     "setup_device.cu": ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"],
     "mesh_device.cu": ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"],
@@ -53,7 +56,7 @@ def _run(cmd: list[str]) -> None:
 def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     """Compiles every source that changed and links the shared library; returns its path."""
     os.makedirs(BUILD, exist_ok=True)
-    headers = [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith(".h")]
+    headers = [os.path.join(CSRC, h) for h in os.listdir(CSRC) if h.endswith((".h", ".cuh"))]
     headers.append(os.path.join(HERE, "..", "include", "solidfem_b200.h"))
     objects, jobs = [], []
     for src, extra in CU_SOURCES.items():
