@@ -435,7 +435,7 @@ sf_status sf_study_system_multiply(sf_study* study, const double* x, double* y);
  * its whole device budget to resident studies, or one that keeps other streams busy, where
  * cudaMalloc can fail and cudaFree waits for the whole device. (sf_study_system_multiply
  * allocates two device buffers per call and copies through the host.) The reduction's scratch is
- * a static 65,792-byte device array in this library, one per device.
+ * a static 262,400-byte device array in this library, one per device.
  *
  * - count at most 8; a larger count is refused with SF_INVALID_ARGUMENT before any work. count 0
  *   does nothing. x, y and energy: 8-byte-aligned device (or managed) memory of the study's

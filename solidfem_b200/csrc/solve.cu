@@ -790,21 +790,22 @@ sf_status solver_read_state(DeviceSolver& s, PcgState* out) {
 // A variant of the conjugate gradient's system product (pcg_spmv_dot_kernel and
 // sell_pcg_spmv_dot_kernel): for each of `count` vectors x_k of caller-owned device memory it
 // writes y_k = A x_k and the energy e_k = x_k . y_k. Rows are summed exactly as the system product
-// sums them; vector k runs in blockIdx.y = k. The reduction's scratch is not the solver's: it is
+// sums them; a SELL system takes all vectors in one walk, a row-group system (under 32,768 rows,
+// resident in L2) vector k in blockIdx.y = k. The reduction's scratch is not the solver's: it is
 // the file-scope array below, whose address is looked up once per device, so a call allocates no
 // memory at all.
 //
-// Scratch layout (g_energy_scratch, 65,792 bytes per device):
+// Scratch layout (g_energy_scratch, 262,400 bytes per device):
 //   bytes [0, 256):   one arrival ticket (unsigned) per vector. Each ticket must be zero when a
 //                     launch starts. Static device storage is zero when the module loads, and the
 //                     last block of each vector puts its ticket back to zero before it exits, so
 //                     the tickets are zero again after every completed call.
-//   bytes [256, ...): kEnergyMaxBlocks partial sums per vector. No initial value is needed: every
+//   bytes [256, ...): kEnergyMaxBlocks slots of partial sums per vector. No initial value is needed: every
 //                     block writes its slot before it takes its ticket.
 // One array serves every study on a device, so two calls whose kernels can run at the same time
 // (different streams, different studies, different host threads) race on it.
 constexpr int kEnergyMaxVectors = 8;
-constexpr int kEnergyMaxBlocks = 1024;  // blocks per vector of one launch
+constexpr int kEnergyMaxBlocks = 4096;  // blocks per vector of one launch
 constexpr size_t kEnergyTicketBytes = 256;
 constexpr size_t kEnergyScratchBytes = kEnergyTicketBytes + (size_t)kEnergyMaxVectors * kEnergyMaxBlocks * sizeof(double);
 constexpr int kEnergyMaxDevices = 64;
@@ -822,17 +823,137 @@ __device__ __forceinline__ void energy_finish(double local, unsigned char* scrat
   if (finish_partials<1>(v, partials, tickets + k, total) && threadIdx.x == 0) energy[k] = total[0];
 }
 
-// SELL-32 system: one thread per row, rows summed as sell_kernel sums them.
-__global__ void __launch_bounds__(kThreads) sell_energy_kernel(SellOp<double> A, const double* __restrict__ x,
-                                                                double* __restrict__ y, uint32_t n,
-                                                                double* __restrict__ energy, unsigned char* scratch) {
-  const size_t off = (size_t)blockIdx.y * n;
+// SELL-32 system, one vector: one thread per row, rows summed as sell_kernel sums them. Bound by
+// the operator's stream: 78 us a call on the gate plate where the walk below takes 83 us with one
+// vector (its blocks finish their energies by themselves, 1,571 partials instead of 786).
+__global__ void __launch_bounds__(kThreads) sell_energy_one_kernel(SellOp<double> A, const double* __restrict__ x,
+                                                                   double* __restrict__ y,
+                                                                   double* __restrict__ energy, unsigned char* scratch) {
   SellDot epi;
-  epi.p = x + off;
-  epi.ap = y + off;
+  epi.p = x;
+  epi.ap = y;
   epi.local = 0.0;
-  sell_rows<double, double, 3, 3, false>(A, x + off, epi, OpenGate{});
+  sell_rows<double, double, 3, 3, false>(A, x, epi, OpenGate{});
   energy_finish(epi.local, scratch, energy);
+}
+
+// SELL-32 system, several vectors: one thread per row and K vectors at once, each row of each vector summed as
+// sell_kernel sums it, so the operator's stream (76 bytes a block) is read from memory once for
+// all the vectors. A block is W slices by G groups of K vectors, a warp each: the G warps of a
+// slice read its stream from L1. The x gathers bound it (3 K loads a block of about 25 sectors,
+// L2 latency), so more than four vectors run as two groups of half the accumulators: 16 warps of
+// K = 4 hide more of it than 8 of K = 8. Gate plate (201,000 rows, 394 MB of operator), 8 vectors:
+// 487 us a call with a grid row per vector (the operator read eight times), 340 us with K = 8 in
+// one thread, 224 us with two groups of four (the floor of its bytes is 72 us); 4 vectors 242 -> 125
+// us, 2 vectors 131 -> 97 us.
+template <int K, int G, int W>
+__global__ void __launch_bounds__(32 * W * G) sell_energy_kernel(SellOp<double> A, const double* __restrict__ x,
+                                                             double* __restrict__ y, uint32_t n, int count,
+                                                             double* __restrict__ energy, unsigned char* scratch) {
+  constexpr int LEN = 9, U = sell_chunk_blocks(LEN, 8), VEC = 2, NV = U * LEN / VEC;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first = (int)(warp / W) * K;  // this warp's vectors: first .. first + K - 1, those below count
+  const double* xg[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) xg[k] = x + (size_t)min(first + k, count - 1) * n;
+  double local[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) local[k] = 0.0;
+  for (uint32_t s = blockIdx.x * W + warp % W; s < A.nslices; s += gridDim.x * W) {
+    const uint32_t slot = s * 32 + lane;
+    const uint32_t row = A.rows[slot], len = A.len[slot], base = A.start[s];
+    double acc[K][3];
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc[k][0] = acc[k][1] = acc[k][2] = 0.0;
+    // Values one chunk ahead, columns two, as in sell_rows.
+    uint32_t cn[U], cf[U];
+    double vn[U * LEN];
+    if (len > 0) {
+      load_cols_shared<U>(A.cols + base + lane * U, cn);
+      const double2* vp = reinterpret_cast<const double2*>(A.vals + (size_t)base * LEN) + lane;
+#pragma unroll
+      for (int q = 0; q < NV; ++q) Vec16<double>::split(__ldg(vp + 32 * q), vn + q * VEC);
+    }
+    if (U < len) load_cols_shared<U>(A.cols + base + 32 * U + lane * U, cf);
+    for (uint32_t k0 = 0; k0 < len; k0 += U) {
+      uint32_t c[U];
+      double v[U * LEN];
+#pragma unroll
+      for (int u = 0; u < U; ++u) c[u] = cn[u];
+#pragma unroll
+      for (int i = 0; i < U * LEN; ++i) v[i] = vn[i];
+      if (k0 + U < len) {
+        const uint32_t q1 = base + 32 * (k0 + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) cn[u] = cf[u];
+        const double2* vp = reinterpret_cast<const double2*>(A.vals + (size_t)q1 * LEN) + lane;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) Vec16<double>::split(__ldg(vp + 32 * q), vn + q * VEC);
+        if (k0 + 2 * U < len) load_cols_shared<U>(A.cols + q1 + 32 * U + lane * U, cf);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (k0 + u >= len) break;
+        double xv[K][3];
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) xv[k][q] = __ldg(xg[k] + (size_t)c[u] * 3 + q);
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+          for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) acc[k][p] += v[u * LEN + p * 3 + q] * xv[k][q];
+      }
+    }
+    if (row < A.nrows)
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (first + k < count)
+#pragma unroll
+          for (int p = 0; p < 3; ++p) {
+            const size_t i = (size_t)row * 3 + p;
+            y[(size_t)(first + k) * n + i] = acc[k][p];
+            local[k] += xg[k][i] * acc[k][p];
+          }
+  }
+  // The energies: each warp's sums by shuffles, the block's slices in order, one partial per
+  // block and vector (vector k's at k * kEnergyMaxBlocks); the last block of the call sums each
+  // vector's partials, a warp per vector, in a fixed order. One ticket (vector 0's) serves the call.
+  __shared__ double sh[K * G][W];
+  __shared__ bool last;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    double v = local[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    if (lane == 0) sh[first + k][warp % W] = v;
+  }
+  __syncthreads();
+  double* partials = reinterpret_cast<double*>(scratch + kEnergyTicketBytes);
+  if ((int)threadIdx.x < count) {
+    double v = sh[threadIdx.x][0];
+#pragma unroll
+    for (int w = 1; w < W; ++w) v += sh[threadIdx.x][w];
+    __stcg(partials + (size_t)threadIdx.x * kEnergyMaxBlocks + blockIdx.x, v);
+    __threadfence();
+  }
+  __syncthreads();
+  unsigned* ticket = reinterpret_cast<unsigned*>(scratch);
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = (int)warp; k < count; k += W * G) {
+    double v = 0.0;
+#pragma unroll 8
+    for (unsigned i = lane; i < gridDim.x; i += 32) v += __ldcg(partials + (size_t)k * kEnergyMaxBlocks + i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    if (lane == 0) energy[k] = v;
+  }
+  if (threadIdx.x == 0) *ticket = 0u;
 }
 
 // Row-group system: LPR lanes per row, rows summed as bsr_kernel sums them.
@@ -876,12 +997,24 @@ sf_status energy_setup(int device, unsigned char** out) {
   return SF_OK;
 }
 
+template <int K, int G>
+void launch_energy_sell(const SellOp<double>& A, const double* x, double* y, uint32_t n, int count, double* energy,
+                        unsigned char* scratch, cudaStream_t st) {
+  // A block per W slices, so the SMs that finish early take the next ones; above the scratch's
+  // slots every block takes the same number of them.
+  constexpr int W = G == 1 ? 4 : 2;  // 128 threads, three resident blocks at about 166 registers
+  const unsigned want = std::max(1u, (A.nslices + W - 1) / W);
+  const unsigned rounds = (want + kEnergyMaxBlocks - 1) / kEnergyMaxBlocks;
+  const unsigned grid = (want + rounds - 1) / rounds;
+  sell_energy_kernel<K, G, W><<<grid, 32 * W * G, 0, st>>>(A, x, y, n, count, energy, scratch);
+}
+
 template <int LPR>
 void launch_energy_lpr(const DevBsr& m, const double* x, double* y, uint32_t n, double* energy, uint64_t count,
                        unsigned char* scratch, cudaStream_t st) {
   Op<double> A = op_of<double>(m);
   Shape sh = shape_of(A, true);
-  dim3 grid((unsigned)std::min(sh.grid, kEnergyMaxBlocks), (unsigned)count);
+  dim3 grid((unsigned)std::min(sh.grid, 1024), (unsigned)count);
   energy_kernel<LPR><<<grid, sh.threads, sh.smem, st>>>(A, x, y, n, energy, scratch);
 }
 
@@ -902,8 +1035,13 @@ sf_status solver_energy_products(DeviceSolver& s, const double* x, double* y, do
   const DevBsr& m = s.system;
   if (m.sell) {
     SellOp<double> A = sell_of<double>(m);
-    dim3 grid((unsigned)std::min(grid_for_slices(m.nslices), kEnergyMaxBlocks), (unsigned)count);
-    sell_energy_kernel<<<grid, kThreads, 0, s.stream>>>(A, x, y, s.n, energy, scratch);
+    const int k = (int)count;
+    if (k == 1) sell_energy_one_kernel<<<std::min(grid_for_slices(m.nslices), 1024), kThreads, 0, s.stream>>>(A, x, y, energy, scratch);
+    else if (k == 2) launch_energy_sell<2, 1>(A, x, y, s.n, k, energy, scratch, s.stream);
+    else if (k == 3) launch_energy_sell<3, 1>(A, x, y, s.n, k, energy, scratch, s.stream);
+    else if (k == 4) launch_energy_sell<4, 1>(A, x, y, s.n, k, energy, scratch, s.stream);
+    else if (k <= 6) launch_energy_sell<3, 2>(A, x, y, s.n, k, energy, scratch, s.stream);
+    else launch_energy_sell<4, 2>(A, x, y, s.n, k, energy, scratch, s.stream);
   } else {
     switch (m.lanes_per_row) {
       case 4: launch_energy_lpr<4>(m, x, y, s.n, energy, count, scratch, s.stream); break;
