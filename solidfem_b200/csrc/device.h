@@ -200,10 +200,14 @@ void pool_setup(int device);
 sf_status setup_inverse_diagonal(cudaStream_t st, uint32_t rows, int rb, const uint32_t* starts, const uint32_t* cols,
                                  const double* vals, double* inv, unsigned long long* bad, double* pivots);
 sf_status setup_block_norms(cudaStream_t st, size_t blocks, int len, const double* vals, double* out);
-// One power step s2 = D^-1 (A v), and v = src / d.
+// One power step s2 = D^-1 (A v); the power iteration's start vector; *norm = the square root of
+// src's squares summed in index order, to the bit, and v = src / *norm, with `scratch` of
+// setup_norm_scratch(n) bytes whose first 256 are zero (they are left zero).
 sf_status setup_power_step(cudaStream_t st, uint32_t rows, int rb, const uint32_t* starts, const uint32_t* cols,
                            const double* vals, const double* inv, const double* v, double* s2);
-sf_status setup_scale(cudaStream_t st, size_t n, const double* src, double d, double* v);
+size_t setup_norm_scratch(size_t n);
+sf_status setup_start_vector(cudaStream_t st, size_t n, double* v);
+sf_status setup_normalize(cudaStream_t st, size_t n, const double* src, void* scratch, double* norm, double* v);
 sf_status setup_entry_rows(cudaStream_t st, uint32_t rows, const uint32_t* starts, uint32_t* out);
 // The geometric strength graph (aggregate.rs:53-69): with out_starts null, each row's strong count
 // into out and its closest squared distance into closest; else the strong columns at out_starts.

@@ -16,7 +16,6 @@
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
-#include <future>
 #include <limits>
 #include <memory>
 
@@ -96,17 +95,6 @@ void symbolic_rows(size_t rows, size_t width, int threads, F&& candidates, vecto
   }
 }
 
-double start_value(size_t index) {  // block.rs:379-382
-  uint64_t mixed = ((uint64_t)index + 1) * 0x9E3779B97F4A7C15ull;
-  return 0.5 + (double)(mixed >> 11) / (double)(1ull << 53);
-}
-
-double norm2(const double* x, size_t n) {  // block.rs:398-404, serial in index order
-  double s = 0.0;
-  for (size_t i = 0; i < n; ++i) s += x[i] * x[i];
-  return std::sqrt(s);
-}
-
 double squared_distance(const vector<P3>& p, size_t a, size_t b) {
   double dx = p[b][0] - p[a][0], dy = p[b][1] - p[a][1], dz = p[b][2] - p[a][2];
   return dx * dx + dy * dy + dz * dz;
@@ -147,19 +135,14 @@ struct SetupMachine {
   Bsr prolongator, ap, coarse;
   sf_status failure = SF_OK;
   bool cancelled = false;
-  // The power iteration needs only the level operator and D^-1, so it runs on a helper thread
-  // from the end of the diagonal phase while this thread builds the strength graph and the
-  // aggregates (host work that touches neither the device nor these buffers); the tentative phase
-  // waits for it before its own device work, the spectral phase takes its result. Declared last,
-  // so it is waited for first.
-  double *power_v = nullptr, *power_s = nullptr;
-  std::future<std::pair<sf_status, double>> power;
+  // The power iteration needs only the level operator and D^-1: it is enqueued in the strength
+  // phase, runs on the device while this thread forms the aggregates, and its result is read in
+  // the spectral phase.
+  double *power_v = nullptr, *power_s = nullptr, *power_norm = nullptr;
+  void* power_scratch = nullptr;
 
   explicit SetupMachine(DeviceSolver& d) : dev(d) {}
-  ~SetupMachine() {
-    if (power.valid()) power.wait();
-    pinned_return(norms);
-  }
+  ~SetupMachine() { pinned_return(norms); }
 
   size_t level_index() const { return levels.size(); }
 
@@ -260,7 +243,6 @@ struct SetupMachine {
     if (!e && blocks) copy_d2h(dev, norms, d_norms, blocks * 8);
     if (!e) e = sync("block norms");
     dev_free(dev, d_norms);
-    if (!e) e = start_power();
     if (e) return e;
     phase = STRENGTH;
     return SF_OK;
@@ -301,12 +283,14 @@ struct SetupMachine {
     if (!e && !strong_cols.empty()) copy_d2h(dev, strong_cols.data(), dcols, strong_cols.size() * 4);
     if (!e) e = sync("strength");
     for (void* p : {(void*)pos, (void*)dclosest, (void*)counts, (void*)dstarts, (void*)dcols}) dev_free(dev, p);
+    if (!e) e = start_power();
     if (!e) phase = AGGREGATE;
     return e;
   }
 
   // Strong neighbours by geometry (aggregate.rs:53-69), two passes so rows run in parallel.
-  void run_strength() {
+  sf_status run_strength() {
+    if (sf_status e = start_power()) return e;  // beside this host work
     size_t rows = current.rows;
     closest.assign(rows, 0.0);
     double limit_scale = reach * reach;
@@ -353,6 +337,7 @@ struct SetupMachine {
         if (strong[at]) strong_cols[w++] = current.cols[at];
     });
     phase = AGGREGATE;
+    return SF_OK;
   }
 
   // Seed, join and sweep passes (aggregate.rs:119-177) then Group (setup_aggregation.rs:165-228).
@@ -434,12 +419,9 @@ struct SetupMachine {
 
   // Tentative prolongator by two-pass Gram-Schmidt per aggregate (transfer.rs:19-68).
   // setup.rs:327-386 on the device (setup_tentative: one thread per aggregate, the host loops'
-  // order and bits). The power iteration shares the stream and the solver's counters, so it is
-  // waited for first; it started at the end of the diagonal phase and has normally finished while
-  // the strength graph and the aggregates were built.
+  // order and bits).
   sf_status run_tentative() {
     const size_t rb = current.rb, rows = current.rows;
-    if (power.valid()) power.wait();
     uint32_t *d_starts = nullptr, *d_members = nullptr;
     sf_status e = SF_OK;
     if (!d_near_null) {  // the finest level's modes come from the host
@@ -463,75 +445,36 @@ struct SetupMachine {
     return SF_OK;
   }
 
-  // Power iteration for lambda_max(D^-1 A) (setup.rs:390-449): the products on the device, the
-  // order-exact norms on the host from a pinned copy of each iterate. Returns the last norm.
-  std::pair<sf_status, double> power_iteration() {
-    cudaSetDevice(dev.device);  // a helper thread starts on device 0
-    const size_t rb = current.rb, rows = current.rows, dofs = rows * rb;
-    double* pinned = (double*)pinned_acquire(std::max<size_t>(1, dofs) * 8);
-    if (!pinned) return {SF_CUDA_ERROR, 0.0};
-    sf_status e = SF_OK;
-    double lm = 0.0;
-    if (dofs) {
-      double* v = power_v;
-      double* s2 = power_s;
-      for (size_t i = 0; i < dofs; ++i) pinned[i] = start_value(i);
-      double n0 = norm2(pinned, dofs);
-      for (size_t i = 0; i < dofs; ++i) pinned[i] /= n0;
-      copy_h2d(dev, v, pinned, dofs * 8);
-      // Each iterate comes back in chunks, each with an event: the host's serial sum of squares
-      // (norm2's order) starts on the first chunk while the rest are still in flight.
-      constexpr int kChunks = 8;
-      cudaEvent_t landed[kChunks];
-      for (int c = 0; c < kChunks; ++c) cudaEventCreateWithFlags(&landed[c], cudaEventDisableTiming);
-      const size_t chunk = (dofs + kChunks - 1) / kChunks;
-      for (int it = 0; it < POWER_ITERATIONS && !e; ++it) {
-        e = setup_power_step(dev.stream, (uint32_t)rows, (int)rb, current.dev_starts, current.dev_cols, current.dev,
-                             inv, v, s2);
-        for (int c = 0; c < kChunks && !e; ++c) {
-          const size_t at = std::min(dofs, c * chunk), len = std::min(dofs, at + chunk) - at;
-          if (len) copy_d2h(dev, pinned + at, s2 + at, len * 8);
-          cudaEventRecord(landed[c], dev.stream);
-        }
-        double sum = 0.0;
-        for (int c = 0; c < kChunks && !e; ++c) {
-          e = cuda_check(cudaEventSynchronize(landed[c]), "power iteration");
-          const size_t at = std::min(dofs, c * chunk), end = std::min(dofs, at + chunk);
-          for (size_t i = at; i < end; ++i) sum += pinned[i] * pinned[i];
-        }
-        if (!e) {
-          double n = std::sqrt(sum);  // norm2 (block.rs:398-404), the same serial sum
-          lm = n;
-          e = setup_scale(dev.stream, dofs, s2, n, v);
-        }
-      }
-      if (!e) e = sync("power iteration");
-      else cudaStreamSynchronize(dev.stream);
-      for (int c = 0; c < kChunks; ++c) cudaEventDestroy(landed[c]);
-    }
-    pinned_return(pinned);  // every copy from it completed at the syncs
-    return {e, lm};
-  }
-
+  // Enqueues the power iteration for lambda_max(D^-1 A) (setup.rs:390-449), once a level: the last
+  // norm stays in power_norm. No host work and no synchronization until the spectral phase.
   sf_status start_power() {
-    const size_t dofs = current.rows * current.rb;
+    if (power_v) return SF_OK;  // a retried aggregation keeps the level's iteration
+    const size_t rb = current.rb, rows = current.rows, dofs = rows * rb;
     sf_status e = dev_alloc(dev, (void**)&power_v, std::max<size_t>(1, dofs) * 8);
     if (!e) e = dev_alloc(dev, (void**)&power_s, std::max<size_t>(1, dofs) * 8);
-    if (e) return e;
-    power = std::async(std::launch::async, [this] { return power_iteration(); });
-    return SF_OK;
+    if (!e) e = dev_alloc(dev, (void**)&power_norm, 8);
+    if (!e) e = dev_alloc(dev, &power_scratch, setup_norm_scratch(dofs));
+    if (!e) e = setup_start_vector(dev.stream, dofs, power_s);
+    if (!e) e = setup_normalize(dev.stream, dofs, power_s, power_scratch, power_norm, power_v);
+    for (int it = 0; it < POWER_ITERATIONS && !e; ++it) {
+      e = setup_power_step(dev.stream, (uint32_t)rows, (int)rb, current.dev_starts, current.dev_cols, current.dev, inv,
+                           power_v, power_s);
+      if (!e) e = setup_normalize(dev.stream, dofs, power_s, power_scratch, power_norm, power_v);
+    }
+    return e;
   }
 
   sf_status run_spectral() {
     const size_t rb = current.rb, rows = current.rows;
-    if (!power.valid())
-      if (sf_status e = start_power()) return e;
-    std::pair<sf_status, double> r = power.get();
-    dev_free(dev, power_v);
-    dev_free(dev, power_s);
-    power_v = power_s = nullptr;
-    if (r.first) return fail(r.first, "the power iteration for the largest eigenvalue failed");
-    lambda_max = r.second * SPECTRAL_MARGIN;
+    if (sf_status e = start_power()) return e;
+    double last = 0.0;
+    if (rows) copy_d2h(dev, &last, power_norm, 8);
+    sf_status e = sync("power iteration");
+    for (void* p : {(void*)power_v, (void*)power_s, (void*)power_norm, power_scratch}) dev_free(dev, p);
+    power_v = power_s = power_norm = nullptr;
+    power_scratch = nullptr;
+    if (e) return e;
+    lambda_max = last * SPECTRAL_MARGIN;
     if (is_coarsest) {
       phase = (rows * rb <= DENSE_LIMIT) ? FACTOR : DONE;
       if (phase == DONE) push_final(false);
@@ -825,7 +768,7 @@ sf_status setup_step(SetupMachine* m, size_t budget, sf_cancel_fn cancel, void* 
         if (m->current.rows >= kDeviceStrengthRows && m->current.dev_starts && m->current.dev_cols)
           s = m->run_strength_device();
         else
-          m->run_strength();
+          s = m->run_strength();
         break;
       case AGGREGATE: m->run_aggregate(); break;
       case TENTATIVE: s = m->run_tentative(); break;

@@ -11,13 +11,12 @@
 // and every sparsity pattern are built on the host (setup.cpp); only values live here.
 //
 // The one sequential reduction, the power iteration's norm (block.rs:398-404 sums the squares in
-// index order), runs on the host (setup.cpp), where a single core adds a dependent chain of
-// doubles several times faster than one GPU thread; the products stay here.
+// index order), runs here too, in parallel and to the bit (norm_terms_kernel).
 #include <cuda_runtime.h>
 
-#include <atomic>
-
 #include <algorithm>
+#include <atomic>
+#include <climits>
 
 #include "device.h"
 
@@ -133,10 +132,204 @@ __global__ void block_norms_kernel(size_t blocks, const double* __restrict__ val
   }
 }
 
-// v = src / d, element by element.
-__global__ void scale_kernel(size_t n, const double* __restrict__ src, double d, double* __restrict__ v) {
+// v = src / d, element by element, d on the device.
+__global__ void scale_kernel(size_t n, const double* __restrict__ src, const double* __restrict__ d,
+                             double* __restrict__ v) {
+  const double by = *d;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    v[i] = src[i] / d;
+    v[i] = src[i] / by;
+}
+
+// The power iteration's start vector (block.rs:379-382).
+__global__ void start_vector_kernel(size_t n, double* __restrict__ v) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const unsigned long long mixed = ((unsigned long long)i + 1) * 0x9E3779B97F4A7C15ull;
+    v[i] = 0.5 + (double)(mixed >> 11) / (double)(1ull << 53);
+  }
+}
+
+// ------------------------------------------------------------ the norm of a serial sum, in parallel
+// s = 0; s = fl(s + fl(x_i x_i)) for i in order; sqrt(s): norm2 (block.rs:398-404) to the bit.
+//
+// While s stays in one binade [2^e, 2^(e+1)), s = m u with u = 2^(e-52) and an integer m, and adding
+// y >= 0 adds an integer to m: floor(y / u), plus one when the fraction is above a half or is a half
+// and m + floor(y / u) is odd (round to nearest, ties to even). So a run of terms is a function of
+// m's parity alone, a pair of increments (for m even, for m odd), and pairs compose associatively:
+// each chunk of 256 terms becomes one pair, computed by a warp, provided the chunk's binade is
+// known. norm_sums_kernel predicts it from an ordinary parallel prefix of the chunk sums;
+// norm_terms_kernel makes the pairs, and its last block walks the chunks in order, 32 at a time,
+// and takes a pair only when s really lies in the predicted binade and stays in it; else it adds
+// the chunk's terms one by one. The prediction therefore decides the time only, never a bit. The
+// serial chunks are the first one and those where s crosses a power of two, about log2(chunks).
+//
+// The walk's dependent additions bound it (one chunk serially is 256 of them, about 1.3 us). On
+// the host this sum took 0.8 ms for the gate plate's 603,000 unknowns, plus the iterate's copy and
+// a synchronization each, 20 times a level.
+constexpr int kNormChunk = 256;   // terms per chunk: eight consecutive ones per lane
+constexpr int kNormThreads = 256;
+constexpr int kNoBinade = INT_MIN;
+
+__device__ __forceinline__ int binade(double s) {
+  const int e = (int)((__double_as_longlong(s) >> 52) & 0x7ff) - 1023;
+  return s > 0.0 && e >= -900 && e <= 900 ? e : kNoBinade;  // no subnormal, infinite or NaN sums
+}
+
+struct Increment {
+  unsigned long long even, odd;
+};
+__device__ __forceinline__ Increment then(const Increment& l, const Increment& r) {
+  Increment t;
+  t.even = l.even + ((l.even & 1) ? r.odd : r.even);
+  t.odd = l.odd + ((l.odd & 1) ? r.even : r.odd);
+  return t;
+}
+
+// True in every thread of the grid's last block to arrive.
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0u;
+  }
+  __syncthreads();
+  __threadfence();
+  return last;
+}
+
+// A warp per chunk: its sum, in any order; then each chunk's binade by the prefix of the sums.
+__global__ void __launch_bounds__(kNormThreads) norm_sums_kernel(size_t n, uint32_t chunks, const double* __restrict__ x,
+                                                                 double* sums, int* __restrict__ binades,
+                                                                 unsigned* ticket) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t c = blockIdx.x * (kNormThreads / 32) + warp;
+  if (c < chunks) {
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < kNormChunk / 32; ++k) {
+      const size_t i = (size_t)c * kNormChunk + 32 * k + lane;
+      const double v = i < n ? x[i] : 0.0;
+      s += v * v;
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) __stcg(sums + c, s);
+  }
+  if (!last_block(ticket)) return;
+  // exclusive prefix: each thread a run of chunks, the threads' totals scanned in shared memory
+  __shared__ double total[kNormThreads];
+  const uint32_t per = (chunks + kNormThreads - 1) / kNormThreads;
+  const uint32_t c0 = min(chunks, threadIdx.x * per), c1 = min(chunks, c0 + per);
+  double mine = 0.0;
+  for (uint32_t k = c0; k < c1; ++k) mine += __ldcg(sums + k);
+  total[threadIdx.x] = mine;
+  __syncthreads();
+  for (int o = 1; o < kNormThreads; o <<= 1) {
+    const double t = threadIdx.x >= o ? total[threadIdx.x - o] : 0.0;
+    __syncthreads();
+    total[threadIdx.x] += t;
+    __syncthreads();
+  }
+  double before = total[threadIdx.x] - mine;
+  if (threadIdx.x == 0) before = 0.0;
+  for (uint32_t k = c0; k < c1; ++k) {
+    const double after = before + __ldcg(sums + k);
+    const int e = binade(before);
+    binades[k] = e == binade(after) ? e : kNoBinade;
+    before = after;
+  }
+}
+
+__global__ void __launch_bounds__(kNormThreads) norm_terms_kernel(size_t n, uint32_t chunks, const double* __restrict__ x,
+                                                                  const int* __restrict__ binades, Increment* pairs,
+                                                                  unsigned* ticket, double* __restrict__ norm) {
+  constexpr int kPer = kNormChunk / 32;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t c = blockIdx.x * (kNormThreads / 32) + warp;
+  if (c < chunks && binades[c] != kNoBinade) {
+    const double scale = __longlong_as_double((long long)(52 - binades[c] + 1023) << 52);  // 1 / u
+    Increment t = {0, 0};
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const size_t i = (size_t)c * kNormChunk + lane * kPer + k;
+      const double v = i < n ? x[i] : 0.0;
+      // y / u exactly (a result below one half may round, and stays below one half); a term past
+      // the binade's end is held at 2^53, which no s in the binade survives.
+      const double q = fmin(v * v * scale, 9007199254740992.0), whole = floor(q), part = q - whole;
+      const unsigned long long m = (unsigned long long)whole;
+      Increment one;
+      one.even = m + (part > 0.5 || (part == 0.5 && (m & 1)) ? 1 : 0);
+      one.odd = m + (part > 0.5 || (part == 0.5 && !(m & 1)) ? 1 : 0);
+      t = then(t, one);
+    }
+    for (int o = 1; o < 32; o <<= 1) {
+      Increment r;
+      r.even = __shfl_down_sync(0xffffffffu, t.even, o);
+      r.odd = __shfl_down_sync(0xffffffffu, t.odd, o);
+      t = then(t, r);
+    }
+    if (lane == 0) {
+      t.even = min(t.even, 1ull << 53);
+      t.odd = min(t.odd, 1ull << 53);
+      __stcg(&pairs[c].even, t.even);
+      __stcg(&pairs[c].odd, t.odd);
+    }
+  }
+  if (!last_block(ticket) || warp != 0) return;
+  __shared__ double y[kNormChunk];
+  double s = 0.0;  // the same in every lane
+  // s after the increment `t`, when it stays in its binade
+  auto advance = [&](const Increment& t) {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(s);
+    const unsigned long long m = (bits & ((1ull << 52) - 1)) | (1ull << 52);
+    const unsigned long long to = m + ((m & 1) ? t.odd : t.even);
+    if (to >> 53) return false;
+    s = __longlong_as_double((long long)((bits & ~((1ull << 52) - 1)) | (to & ((1ull << 52) - 1))));
+    return true;
+  };
+  for (uint32_t b = 0; b < chunks; b += 32) {
+    const uint32_t mine = b + lane;
+    int e = kNoBinade;
+    Increment p = {0, 0};
+    if (mine < chunks) {
+      e = __ldg(binades + mine);
+      if (e != kNoBinade) {
+        p.even = __ldcg(&pairs[mine].even);
+        p.odd = __ldcg(&pairs[mine].odd);
+      }
+    }
+    const int now = binade(s);
+    if (now != kNoBinade && __all_sync(0xffffffffu, mine >= chunks || e == now)) {
+      Increment t = p;
+      for (int o = 1; o < 32; o <<= 1) {
+        Increment r;
+        r.even = __shfl_down_sync(0xffffffffu, t.even, o);
+        r.odd = __shfl_down_sync(0xffffffffu, t.odd, o);
+        t = then(t, r);
+      }
+      t.even = __shfl_sync(0xffffffffu, t.even, 0);
+      t.odd = __shfl_sync(0xffffffffu, t.odd, 0);
+      if (advance(t)) continue;
+    }
+    for (int j = 0; j < 32 && b + j < chunks; ++j) {
+      Increment t;
+      t.even = __shfl_sync(0xffffffffu, p.even, j);
+      t.odd = __shfl_sync(0xffffffffu, p.odd, j);
+      const int ej = __shfl_sync(0xffffffffu, e, j);
+      if (ej != kNoBinade && ej == binade(s) && advance(t)) continue;
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < kPer; ++k) {
+        const size_t i = (size_t)(b + j) * kNormChunk + 32 * k + lane;
+        const double v = i < n ? x[i] : 0.0;
+        y[32 * k + lane] = v * v;  // adding the zeros past the end changes nothing
+      }
+      __syncwarp();
+#pragma unroll 16
+      for (int i = 0; i < kNormChunk; ++i) s += y[i];
+    }
+  }
+  if (lane == 0) *norm = sqrt(s);
 }
 
 // s2 = D^-1 (A v) for one block row per thread, in the order of setup.rs:404-432.
@@ -752,10 +945,29 @@ sf_status setup_power_step(cudaStream_t st, uint32_t rows, int rb, const uint32_
   return cuda_check(cudaGetLastError(), "power step");
 }
 
-sf_status setup_scale(cudaStream_t st, size_t n, const double* src, double d, double* v) {
+size_t setup_norm_scratch(size_t n) {
+  const size_t chunks = (n + kNormChunk - 1) / kNormChunk;
+  return 256 + chunks * (sizeof(Increment) + 8 + 4);
+}
+
+sf_status setup_start_vector(cudaStream_t st, size_t n, double* v) {
   if (n == 0) return SF_OK;
-  scale_kernel<<<grid_for(n), kT, 0, st>>>(n, src, d, v);
-  return cuda_check(cudaGetLastError(), "scale");
+  start_vector_kernel<<<grid_for(n), kT, 0, st>>>(n, v);
+  return cuda_check(cudaGetLastError(), "start vector");
+}
+
+sf_status setup_normalize(cudaStream_t st, size_t n, const double* src, void* scratch, double* norm, double* v) {
+  if (n == 0) return SF_OK;
+  const uint32_t chunks = (uint32_t)((n + kNormChunk - 1) / kNormChunk);
+  unsigned* tickets = (unsigned*)scratch;
+  Increment* pairs = (Increment*)((char*)scratch + 256);
+  double* sums = (double*)(pairs + chunks);
+  int* binades = (int*)(sums + chunks);
+  const unsigned grid = (chunks + kNormThreads / 32 - 1) / (kNormThreads / 32);
+  norm_sums_kernel<<<grid, kNormThreads, 0, st>>>(n, chunks, src, sums, binades, tickets);
+  norm_terms_kernel<<<grid, kNormThreads, 0, st>>>(n, chunks, src, binades, pairs, tickets + 1, norm);
+  scale_kernel<<<grid_for(n), kT, 0, st>>>(n, src, norm, v);
+  return cuda_check(cudaGetLastError(), "normalize");
 }
 
 sf_status setup_union_rows(cudaStream_t st, uint32_t rows, uint32_t width, const uint32_t* outer_starts,
