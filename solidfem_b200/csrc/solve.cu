@@ -29,7 +29,7 @@ void launch_pcg_spmv_lpr(DeviceSolver& s) {
   Op<double> A = op_of<double>(s.system);
   Shape sh = shape_of(A, true);
   launch_body<pcg_spmv_dot_kernel<LPR>>(sh.grid, sh.threads, sh.smem, s.stream, A, s.p, s.ap, s.partials, s.state);
-  launch_body<pcg_update_kernel>(kReduceBlocks, kReduceThreads, 0, s.stream, s.n, s.p, s.ap, s.x, s.r, s.partials, s.state);
+  launch_body<pcg_update_kernel>(grid_for_reduction(s.n), kReduceThreads, 0, s.stream, s.n, s.p, s.ap, s.x, s.r, s.partials, s.state);
   launch_body<pcg_check_kernel<LPR>>(sh.grid, sh.threads, sh.smem, s.stream, A, s.x, s.rhs, s.r, s.partials, s.state);
 }
 
@@ -511,7 +511,7 @@ sf_status solver_init_pcg(DeviceSolver& s, double tolerance, uint64_t max_iterat
   copy_h2d(s, s.state, &h, sizeof(h));
   int one_active = ST_ACTIVE;
   copy_h2d(s, s.always_active, &one_active, sizeof(int));
-  launch_body<pcg_init_kernel>(kReduceBlocks, kReduceThreads, 0, s.stream, s.n, s.rhs, s.x, s.r, s.partials, s.state);
+  launch_body<pcg_init_kernel>(grid_for_reduction(s.n), kReduceThreads, 0, s.stream, s.n, s.rhs, s.x, s.r, s.partials, s.state);
   return solver_enqueue_reset(s);
 }
 
@@ -519,10 +519,10 @@ sf_status solver_enqueue_reset(DeviceSolver& s) {
   const int* status = &s.state->status;
   enqueue_precondition(s, s.r, s.z, s.z32, status);
   if (s.vector_single && s.multigrid) {
-    launch_body<pcg_dot_rz_kernel<float>>(kReduceBlocks, kReduceThreads, 0, s.stream, s.n, s.r, s.z32, s.ap, s.partials, s.state);
+    launch_body<pcg_dot_rz_kernel<float>>(grid_for_reduction(s.n), kReduceThreads, 0, s.stream, s.n, s.r, s.z32, s.ap, s.partials, s.state);
     launch_body<pcg_update_p_kernel<float>>(grid_for_elems(s.n), kThreads, 0, s.stream, s.n, s.z32, s.p, s.state);
   } else {
-    launch_body<pcg_dot_rz_kernel<double>>(kReduceBlocks, kReduceThreads, 0, s.stream, s.n, s.r, s.z, s.ap, s.partials, s.state);
+    launch_body<pcg_dot_rz_kernel<double>>(grid_for_reduction(s.n), kReduceThreads, 0, s.stream, s.n, s.r, s.z, s.ap, s.partials, s.state);
     launch_body<pcg_update_p_kernel<double>>(grid_for_elems(s.n), kThreads, 0, s.stream, s.n, s.z, s.p, s.state);
   }
   s.launches_per_iteration += 2;
@@ -537,7 +537,7 @@ sf_status solver_enqueue_iteration(DeviceSolver& s) {
     SellOp<double> A = sell_of<double>(s.system);
     int grid = std::min(grid_for_slices(s.system.nslices), kReduceBlocks * 2);
     launch_body<sell_pcg_spmv_dot_kernel>(grid, kThreads, 0, st, A, s.p, s.ap, s.partials, s.state);
-    launch_body<pcg_update_kernel>(kReduceBlocks, kReduceThreads, 0, st, s.n, s.p, s.ap, s.x, s.r, s.partials, s.state);
+    launch_body<pcg_update_kernel>(grid_for_reduction(s.n), kReduceThreads, 0, st, s.n, s.p, s.ap, s.x, s.r, s.partials, s.state);
     launch_body<sell_pcg_check_kernel>(grid, kThreads, 0, st, A, s.x, s.rhs, s.r, s.partials, s.state);
   } else switch (s.system.lanes_per_row) {
     case 8: launch_pcg_spmv_lpr<8>(s); break;
@@ -547,10 +547,10 @@ sf_status solver_enqueue_iteration(DeviceSolver& s) {
   s.launches_per_iteration += 3;
   enqueue_precondition(s, s.r, s.z, s.z32, status);
   if (s.vector_single && s.multigrid) {
-    launch_body<pcg_dot_rz_kernel<float>>(kReduceBlocks, kReduceThreads, 0, st, s.n, s.r, s.z32, s.ap, s.partials, s.state);
+    launch_body<pcg_dot_rz_kernel<float>>(grid_for_reduction(s.n), kReduceThreads, 0, st, s.n, s.r, s.z32, s.ap, s.partials, s.state);
     launch_body<pcg_update_p_kernel<float>>(grid_for_elems(s.n), kThreads, 0, st, s.n, s.z32, s.p, s.state);
   } else {
-    launch_body<pcg_dot_rz_kernel<double>>(kReduceBlocks, kReduceThreads, 0, st, s.n, s.r, s.z, s.ap, s.partials, s.state);
+    launch_body<pcg_dot_rz_kernel<double>>(grid_for_reduction(s.n), kReduceThreads, 0, st, s.n, s.r, s.z, s.ap, s.partials, s.state);
     launch_body<pcg_update_p_kernel<double>>(grid_for_elems(s.n), kThreads, 0, st, s.n, s.z, s.p, s.state);
   }
   s.launches_per_iteration += 2;

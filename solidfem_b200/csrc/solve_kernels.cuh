@@ -38,13 +38,20 @@ const uint32_t kGroupTarget = 4096;     // value bytes a row group aims at
 const int kSmemPerBlockTarget = 72 * 1024;
 
 // ------------------------------------------------------------ programmatic dependent launch
-// Every solve kernel is launched with programmatic stream serialization: its launch is prepared
-// while the predecessor runs, and at entry it waits until the predecessor grid has completed and
-// its writes are visible (griddepcontrol.wait). The data dependence is unchanged; without a
-// programmatic predecessor the wait returns at once.
-__device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
+// Every solve kernel is launched with programmatic stream serialization. A body first requests what
+// no solve kernel ever writes (its first operator loads, D^-1), then calls pdl_wait(): it waits
+// until the predecessor grid has completed and its writes are visible (griddepcontrol.wait), and
+// from there lets the successor's blocks start (griddepcontrol.launch_dependents) and do the same.
+// So at most the next kernel's blocks sit beside a running grid, each with its first operator loads
+// in flight, and a launch's start no longer adds its own latency to the chain. What a predecessor
+// writes is read after the wait with plain loads, never through the read-only path (ld.global.nc),
+// whose lines may be older than the wait. Every thread of a grid waits, so grids complete in order.
+// Without a programmatic predecessor the wait returns at once.
+// @PDLFIGURES@
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+constexpr uint32_t kOneWave = kReduceBlocks * kReduceThreads;  // unknowns the vector kernels take one per thread
+constexpr uint32_t kOneWaveRows = kOneWave / 3;
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 
 // ------------------------------------------------------------ kernel bodies and batched launches
@@ -84,12 +91,10 @@ __device__ __forceinline__ void apply_pack(const Pack<H, T...>& p, Done... done)
 
 template <auto Body, typename... P>
 __global__ void __launch_bounds__(kThreads) single_kernel(P... args) {
-  pdl_enter();
   Body(args...);
 }
 template <auto Body, typename PackT>
 __global__ void __launch_bounds__(kThreads) batched_kernel(const PackT* __restrict__ table) {
-  pdl_enter();
   const PackT a = table[blockIdx.y];
   apply_pack<Body>(a);
 }
@@ -97,12 +102,12 @@ __global__ void __launch_bounds__(kThreads) batched_kernel(const PackT* __restri
 // The same wrappers for a body launched with `Threads` threads per block (the coarse tail).
 template <auto Body, int Threads, typename... P>
 __global__ void __launch_bounds__(Threads) single_kernel_n(P... args) {
-  pdl_enter();
+  pdl_wait();
   Body(args...);
 }
 template <auto Body, int Threads, typename PackT>
 __global__ void __launch_bounds__(Threads) batched_kernel_n(const PackT* __restrict__ table) {
-  pdl_enter();
+  pdl_wait();
   const PackT a = table[blockIdx.y];
   apply_pack<Body>(a);
 }
@@ -275,38 +280,55 @@ __host__ __device__ __forceinline__ uint32_t slot_bytes(const Op<S>& A) {
   return A.vbuf + A.cbuf + A.sbuf;
 }
 
-// Gates: the row walks (run_groups, sell_rows, split_rows) test their kernel's gate (the status
-// word) only after their first operator loads have been requested, so the status load and those
-// loads travel together instead of one after the other. The operator arrays are never written by
-// a solve kernel, and a closed gate ends the walk before any x gather, epilogue load or store.
-// sell_rows' and split_rows' row-map loads are volatile so the compiler keeps them ahead of the
-// gate's branch.
+// Gates: a row walk (run_groups, sell_rows, split_rows) loads its kernel's gate (the status word)
+// after pdl_wait() and tests it once its first x gathers are requested, so the word and the gathers
+// travel together; a closed gate ends the walk before any store. An eager gate (the usual, open
+// one) lets the walk request its first operator loads before pdl_wait(); the operator arrays are
+// never written by a solve kernel. ld_early's loads are volatile so the compiler keeps them there.
 __device__ __forceinline__ uint32_t ld_early(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
   return v;
 }
 
-// load() reads the gate's word(s); open() tests them. run_groups issues the load before its first
-// operator loads and tests it after them; gate() does both at once.
+// A gather of a vector the predecessor wrote: a plain (not read-only path) load that the compiler
+// may still schedule freely among the walk's other loads. after_wait() redefines the vector's
+// pointer, so that no load through it can be moved above the pdl_wait() before it.
+__device__ __forceinline__ float ld_x(const float* p) {
+  float v;
+  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double ld_x(const double* p) {
+  double v;
+  asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+template <typename V>
+__device__ __forceinline__ const V* after_wait(const V* p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+
+// load() reads the gate's word(s); open() tests them.
 struct StatusGate {
+  static constexpr bool kEager = true;
   const int* status;
   __device__ __forceinline__ int load() const { return *status; }
   __device__ __forceinline__ static bool open(int w) { return w == ST_ACTIVE; }
-  __device__ __forceinline__ bool operator()() const { return open(load()); }
 };
 struct OpenGate {
+  static constexpr bool kEager = true;
   __device__ __forceinline__ int load() const { return 0; }
   __device__ __forceinline__ static bool open(int) { return true; }
-  __device__ __forceinline__ bool operator()() const { return true; }
 };
 
-// The true-residual check runs only in its mode.
+// The true-residual check runs only in its mode, rarely: nothing is requested before its test.
 struct CheckGate {
+  static constexpr bool kEager = false;
   const PcgState* st;
   __device__ __forceinline__ int2 load() const { return make_int2(st->status, st->mode); }
   __device__ __forceinline__ static bool open(int2 w) { return w.x == ST_ACTIVE && w.y == MODE_CHECK; }
-  __device__ __forceinline__ bool operator()() const { return open(load()); }
 };
 
 // Walks this warp's row groups. Per row (one team of LPR lanes each) it calls epi.pre(row, live,
@@ -342,17 +364,19 @@ __device__ __forceinline__ bool run_groups(const Op<S>& A, const V* __restrict__
     }
   };
   const uint4 none = make_uint4(0, 0, 0, 0);
-  // The gate's load goes first (the staging asm below is a compiler memory barrier) and is tested
-  // once the first group's staging is in flight; a closed gate drains the copies and ends.
-  const auto word = gate.load();
+  if constexpr (!Gate::kEager) {
+    pdl_wait();
+    if (!Gate::open(gate.load())) return false;
+  }
   uint4 cur = g < A.ngroups ? A.groups[g] : none;
   uint4 nxt = g + nw < A.ngroups ? A.groups[g + nw] : none;
   if (g < A.ngroups) issue(cur, 0);
   cp_async_commit();
-  if (!Gate::open(word)) {
-    cp_async_wait_all();
-    return false;
-  }
+  if constexpr (Gate::kEager) pdl_wait();
+  pdl_release();
+  const V* const xp = after_wait(x);
+  const auto word = gate.load();
+  bool tested = !Gate::kEager;
   for (int k = 0; g < A.ngroups; ++k, g += nw) {
     const int slot = k & 1;
     const bool has_next = g + nw < A.ngroups;
@@ -374,39 +398,54 @@ __device__ __forceinline__ bool run_groups(const Op<S>& A, const V* __restrict__
       V acc[RB], mag[RB];
 #pragma unroll
       for (int p = 0; p < RB; ++p) acc[p] = mag[p] = V(0);
+      uint32_t j = 0, b1 = 0;
       if (live) {
-        const uint32_t b0 = rst[lr] - cur.z, b1 = rst[lr + 1] - cur.z;
-        for (uint32_t j = b0 + tl; j < b1; j += 2 * LPR) {
-          const uint32_t j2 = j + LPR;
-          const bool two = j2 < b1;
-          const uint32_t c0 = cols[j], c1 = two ? cols[j2] : c0;
-          V xa[CB], xb[CB];
+        j = rst[lr] - cur.z + tl;
+        b1 = rst[lr + 1] - cur.z;
+      }
+      V xa[CB], xb[CB];
+      auto gather = [&]() {
+        const uint32_t j2 = j + LPR;
+        const uint32_t c0 = cols[j], c1 = j2 < b1 ? cols[j2] : c0;
+#pragma unroll
+        for (int q = 0; q < CB; ++q) {
+          xa[q] = ld_x(xp + (size_t)c0 * CB + q);
+          xb[q] = ld_x(xp + (size_t)c1 * CB + q);
+        }
+      };
+      if (j < b1) gather();
+      if (!tested) {  // uniform over the grid
+        if (!Gate::open(word)) {
+          cp_async_wait_all();
+          return false;
+        }
+        tested = true;
+      }
+      while (j < b1) {
+        const uint32_t j2 = j + LPR;
+        const bool two = j2 < b1;
+        const S* ba = vals + (size_t)j * LEN;
+        const S* bb = vals + (size_t)(two ? j2 : j) * LEN;
+#pragma unroll
+        for (int p = 0; p < RB; ++p)
 #pragma unroll
           for (int q = 0; q < CB; ++q) {
-            xa[q] = __ldg(x + (size_t)c0 * CB + q);
-            xb[q] = __ldg(x + (size_t)c1 * CB + q);
+            V t = V(ba[p * CB + q]) * xa[q];
+            acc[p] += t;
+            if (MAG) mag[p] += fabs(t);
           }
-          const S* ba = vals + (size_t)j * LEN;
-          const S* bb = vals + (size_t)(two ? j2 : j) * LEN;
+        if (two) {
 #pragma unroll
           for (int p = 0; p < RB; ++p)
 #pragma unroll
             for (int q = 0; q < CB; ++q) {
-              V t = V(ba[p * CB + q]) * xa[q];
+              V t = V(bb[p * CB + q]) * xb[q];
               acc[p] += t;
               if (MAG) mag[p] += fabs(t);
             }
-          if (two) {
-#pragma unroll
-            for (int p = 0; p < RB; ++p)
-#pragma unroll
-              for (int q = 0; q < CB; ++q) {
-                V t = V(bb[p * CB + q]) * xb[q];
-                acc[p] += t;
-                if (MAG) mag[p] += fabs(t);
-              }
-          }
         }
+        j += 2 * LPR;
+        if (j < b1) gather();
       }
       __syncwarp();
 #pragma unroll
@@ -423,7 +462,7 @@ __device__ __forceinline__ bool run_groups(const Op<S>& A, const V* __restrict__
     nxt = after;
   }
   cp_async_wait_all();
-  return true;
+  return tested || Gate::open(word);
 }
 
 template <typename V, int RB>
@@ -567,6 +606,8 @@ __device__ __forceinline__ void cheb_start_kernel(uint32_t rows, const S* __rest
                                                                V* __restrict__ r, V* __restrict__ d,
                                                                V* __restrict__ x, V theta,
                                                                const int* __restrict__ status) {
+  pdl_wait();
+  if (rows <= kOneWaveRows) pdl_release();
   if (*status != ST_ACTIVE) return;
   for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += gridDim.x * blockDim.x) {
     size_t base = (size_t)row * RB;
@@ -591,6 +632,7 @@ __device__ __forceinline__ void cheb_start_kernel(uint32_t rows, const S* __rest
 
 template <typename V>
 __device__ __forceinline__ void add_kernel(size_t n, V* __restrict__ x, const V* __restrict__ y, const int* __restrict__ status) {
+  pdl_wait();
   if (*status != ST_ACTIVE) return;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     x[i] = x[i] + y[i];
@@ -598,6 +640,7 @@ __device__ __forceinline__ void add_kernel(size_t n, V* __restrict__ x, const V*
 
 template <typename B, typename V>
 __device__ __forceinline__ void convert_kernel(size_t n, const B* __restrict__ in, V* __restrict__ out, const int* __restrict__ status) {
+  pdl_wait();
   if (*status != ST_ACTIVE) return;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     out[i] = V(in[i]);
@@ -609,15 +652,29 @@ template <typename V>
 __device__ __forceinline__ void coarse_solve_kernel(uint32_t n, const double* __restrict__ inv,
                                                                  const V* __restrict__ b, V* __restrict__ x,
                                                                  const int* __restrict__ status) {
-  if (*status != ST_ACTIVE) return;
+  constexpr int kAhead = 4;  // entries of its row each lane requests before it waits for b
   int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  bool waited = false;
   for (uint32_t row = blockIdx.x * kWarps + warp; row < n; row += gridDim.x * kWarps) {
     const double* a = inv + (size_t)row * n;
+    double av[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) av[k] = lane + 32u * k < n ? a[lane + 32 * k] : 0.0;
+    if (!waited) {
+      pdl_wait();
+      pdl_release();
+      if (*status != ST_ACTIVE) return;
+      waited = true;
+    }
     double s = 0.0;
-    for (uint32_t j = lane; j < n; j += 32) s += __ldg(a + j) * (double)b[j];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k)
+      if (lane + 32u * k < n) s += av[k] * (double)b[lane + 32 * k];
+    for (uint32_t j = lane + 32 * kAhead; j < n; j += 32) s += a[j] * (double)b[j];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
     if (lane == 0) x[row] = V(s);
   }
+  if (!waited) pdl_wait();
 }
 
 // ------------------------------------------------------------ fixed-order reductions
@@ -745,6 +802,7 @@ __device__ __forceinline__ bool sell_rows(const SellOp<S>& A, const V* __restric
   constexpr int NV = U * LEN / VEC;
   static_assert((U * LEN) % VEC == 0, "a lane chunk is whole 16-byte vectors");
   typedef typename Vec16<S>::type W;
+  pdl_wait();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = blockDim.x >> 5;
   bool open = false;
@@ -754,7 +812,7 @@ __device__ __forceinline__ bool sell_rows(const SellOp<S>& A, const V* __restric
     const uint32_t n = ld_early(A.len + slot);
     const uint32_t base = ld_early(A.start + s);
     if (!open) {
-      if (!gate()) return false;
+      if (!Gate::open(gate.load())) return false;
       open = true;
     }
     const bool live = row < A.nrows;
@@ -797,7 +855,7 @@ __device__ __forceinline__ bool sell_rows(const SellOp<S>& A, const V* __restric
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int q = 0; q < CB; ++q) xv[u][q] = k0 + u < n ? __ldg(x + (size_t)c[u] * CB + q) : V(0);
+        for (int q = 0; q < CB; ++q) xv[u][q] = k0 + u < n ? ld_x(x + (size_t)c[u] * CB + q) : V(0);
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         if (k0 + u >= n) break;
@@ -813,7 +871,7 @@ __device__ __forceinline__ bool sell_rows(const SellOp<S>& A, const V* __restric
     }
     epi.post(row, live, n, acc, mag);
   }
-  return open || gate();
+  return open || Gate::open(gate.load());
 }
 
 template <typename V, int RB, int OP>
@@ -939,6 +997,7 @@ __device__ __forceinline__ bool split_rows(const SellOp<S>& A, const V* __restri
   constexpr int NV = U * CB / VEC;
   static_assert((U * CB) % VEC == 0, "a lane chunk is whole 16-byte vectors");
   typedef typename Vec16<S>::type W;
+  pdl_wait();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t m = lane / 6, part = lane - 6 * m;
   const uint32_t warps = blockDim.x >> 5;
@@ -949,7 +1008,7 @@ __device__ __forceinline__ bool split_rows(const SellOp<S>& A, const V* __restri
     const uint32_t n = ld_early(A.len + slot);
     const uint32_t base = ld_early(A.start + s);
     if (!open) {
-      if (!gate()) return false;
+      if (!Gate::open(gate.load())) return false;
       open = true;
     }
     const bool live = row < A.nrows;
@@ -985,7 +1044,7 @@ __device__ __forceinline__ bool split_rows(const SellOp<S>& A, const V* __restri
 #pragma unroll
       for (int u = 0; u < U; ++u)
 #pragma unroll
-        for (int q = 0; q < CB; ++q) xv[u][q] = k0 + u < n ? __ldg(x + (size_t)c[u] * CB + q) : V(0);
+        for (int q = 0; q < CB; ++q) xv[u][q] = k0 + u < n ? ld_x(x + (size_t)c[u] * CB + q) : V(0);
       V bs[U];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
@@ -1001,7 +1060,7 @@ __device__ __forceinline__ bool split_rows(const SellOp<S>& A, const V* __restri
     }
     epi.post(row, part, live, acc);
   }
-  return open || gate();
+  return open || Gate::open(gate.load());
 }
 
 template <typename V, int OP>
@@ -1865,6 +1924,8 @@ __device__ __forceinline__ void pcg_spmv_dot_kernel(Op<double> A, const double* 
 __device__ __forceinline__ void pcg_update_kernel(uint32_t n, const double* __restrict__ p,
                                                                const double* __restrict__ ap, double* __restrict__ x,
                                                                double* __restrict__ r, double* partials, PcgState* st) {
+  pdl_wait();
+  if (n <= kOneWave) pdl_release();
   if (st->status != ST_ACTIVE) return;
   double alpha = st->alpha, na = -alpha;
   double local = 0.0;
@@ -1968,6 +2029,8 @@ template <typename Z>
 __device__ __forceinline__ void pcg_dot_rz_kernel(uint32_t n, const double* __restrict__ r,
                                                                const Z* __restrict__ z, const double* __restrict__ ap,
                                                                double* partials, PcgState* st) {
+  pdl_wait();
+  if (n <= kOneWave) pdl_release();
   if (st->status != ST_ACTIVE) return;
   bool flex = st->flexible && st->mode == MODE_NORMAL;
   double rz = 0.0, apz = 0.0;
@@ -2007,6 +2070,8 @@ __device__ __forceinline__ void pcg_dot_rz_kernel(uint32_t n, const double* __re
 // p = z + beta p, or p = z after a restart.
 template <typename Z>
 __device__ __forceinline__ void pcg_update_p_kernel(uint32_t n, const Z* __restrict__ z, double* __restrict__ p, PcgState* st) {
+  pdl_wait();
+  if (n <= kOneWave) pdl_release();
   if (st->status != ST_ACTIVE) return;
   bool restart = st->mode == MODE_RESTART;
   double beta = st->beta;
@@ -2032,6 +2097,7 @@ __device__ __forceinline__ void pcg_update_p_kernel(uint32_t n, const Z* __restr
 // Initial state (Pcg::new, pcg.rs:135-164): x = 0, r = b, rhs norm; then reset_direction.
 __device__ __forceinline__ void pcg_init_kernel(uint32_t n, const double* __restrict__ b, double* __restrict__ x,
                                                              double* __restrict__ r, double* partials, PcgState* st) {
+  pdl_wait();
   double local = 0.0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     x[i] = 0.0;
@@ -2051,6 +2117,8 @@ __device__ __forceinline__ void pcg_init_kernel(uint32_t n, const double* __rest
 // Jacobi: z = r / diag (preconditioner.rs:237-247), stored as the inverse diagonal.
 __device__ __forceinline__ void jacobi_kernel(uint32_t n, const double* __restrict__ inv, const double* __restrict__ r,
                               double* __restrict__ z, const int* __restrict__ status) {
+  pdl_wait();
+  if (n <= kOneWave) pdl_release();
   if (*status != ST_ACTIVE) return;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) z[i] = r[i] * inv[i];
 }
@@ -2079,6 +2147,13 @@ int grid_for_rows(size_t rows) {
   return (int)std::max<size_t>(1, std::min(blocks, (size_t)sm_count() * 8));
 }
 
+// Blocks of a fixed-order reduction over n elements: no more than have an element. The blocks left
+// out would add exact zeros at the end of each thread's partials, so the sums keep their bits;
+// they cost the last block's wait for 592 arrivals on one ticket (n = 9,720: 38 blocks).
+int grid_for_reduction(size_t n) {
+  return (int)std::max<size_t>(1, std::min<size_t>((n + kReduceThreads - 1) / kReduceThreads, kReduceBlocks));
+}
+
 // Launch shape of a grouped product: warps per block so a block stages at most about 72 KB, and
 // a grid of whole waves (resident blocks per SM times SMs), never more warps than groups.
 struct Shape {
@@ -2095,7 +2170,7 @@ Shape shape_of(const Op<S>& A, bool reduction) {
   int per_sm = (int)std::max<size_t>(1, std::min<size_t>(2048 / (32 * warps), (228 * 1024) / (smem + 1024)));
   size_t want = (A.ngroups + warps - 1) / warps;
   size_t grid = std::min<size_t>(want, (size_t)sm_count() * per_sm);
-  if (reduction) grid = std::min<size_t>((size_t)sm_count() * per_sm, (size_t)kReduceBlocks * 2);
+  if (reduction) grid = std::min<size_t>(grid, (size_t)kReduceBlocks * 2);
   return {32 * warps, (int)std::max<size_t>(1, grid), smem};
 }
 
@@ -2114,10 +2189,13 @@ void launch_bsr_lpr(const DevBsr& m, const V* x, V* y, const V* b, const int* st
 // evenly instead of two eight-warp blocks on some SMs and one on others (mixed solve 182.5 ->
 // 181.7 ms). Same bits; FP64 unchanged.
 constexpr int kSellThreads = 64;
-inline int sell_threads() { return kSellThreads; }
 inline int sell_grid(uint32_t nslices) {
   const int w = kSellThreads / 32;
   return (int)std::max<size_t>(1, (nslices + w - 1) / w);
+}
+template <auto Body, typename... A>
+void launch_walk(uint32_t nslices, cudaStream_t st, A&&... args) {
+  launch_body<Body>(sell_grid(nslices), kSellThreads, 0, st, std::forward<A>(args)...);
 }
 
 int grid_for_slices(uint32_t nslices) {
@@ -2127,7 +2205,7 @@ int grid_for_slices(uint32_t nslices) {
 
 template <typename S, typename V, int RB, int CB, int OP>
 void launch_sell(const DevBsr& m, const V* x, V* y, const V* b, const int* status, cudaStream_t st) {
-  launch_body<sell_kernel<S, V, RB, CB, OP>>(sell_grid(m.nslices), sell_threads(), 0, st, sell_of<S>(m), x, y, b, status);
+  launch_walk<sell_kernel<S, V, RB, CB, OP>>(m.nslices, st, sell_of<S>(m), x, y, b, status);
 }
 
 template <typename S, typename V, int RB, int CB, int OP>
@@ -2147,9 +2225,9 @@ void launch_bsr(const DevBsr& m, const V* x, V* y, const V* b, const int* status
 template <typename S, typename V, int OP>
 void launch_split(const DevBsr& m, const V* x, V* y, const V* b, const int* status, cudaStream_t st) {
   if (m.cb == 3)
-    launch_body<split_kernel<S, V, 3, OP>>(sell_grid(m.nslices), sell_threads(), 0, st, sell_of<S>(m), x, y, b, status);
+    launch_walk<split_kernel<S, V, 3, OP>>(m.nslices, st, sell_of<S>(m), x, y, b, status);
   else
-    launch_body<split_kernel<S, V, 6, OP>>(sell_grid(m.nslices), sell_threads(), 0, st, sell_of<S>(m), x, y, b, status);
+    launch_walk<split_kernel<S, V, 6, OP>>(m.nslices, st, sell_of<S>(m), x, y, b, status);
 }
 
 template <typename S, typename V, int RB, int OP>
@@ -2186,14 +2264,13 @@ void launch_cheb_step(const DevLevel& L, const V* d_old, V* d_new, V* r, V* x, V
                       const int* status, cudaStream_t st) {
   if constexpr (RB == 6) {
     if (L.a.split) {
-      launch_body<split_cheb_kernel<S, V>>(sell_grid(L.a.nslices), sell_threads(), 0, st, sell_of<S>(L.a),
+      launch_walk<split_cheb_kernel<S, V>>(L.a.nslices, st, sell_of<S>(L.a),
                                            (const S*)L.dinv, d_old, d_new, r, x, outer, (V)keep, (V)step, status);
       return;
     }
   }
   if (L.a.sell) {
-    launch_body<sell_cheb_kernel<S, V, RB>>(sell_grid(L.a.nslices), sell_threads(), 0, st,
-        sell_of<S>(L.a), (const S*)L.dinv, d_old, d_new, r, x, outer, (V)keep, (V)step, status);
+    launch_walk<sell_cheb_kernel<S, V, RB>>(L.a.nslices, st, sell_of<S>(L.a), (const S*)L.dinv, d_old, d_new, r, x, outer, (V)keep, (V)step, status);
     return;
   }
   switch (L.a.lanes_per_row) {
@@ -2218,13 +2295,13 @@ void launch_start_rb(const DevBsr& m, const V* x, const V* b, const StartArgs<S,
                      cudaStream_t st) {
   if constexpr (RB == 6) {
     if (m.split) {
-      launch_body<split_start_kernel<S, V, CB, OP>>(sell_grid(m.nslices), sell_threads(), 0, st, sell_of<S>(m), x, b,
+      launch_walk<split_start_kernel<S, V, CB, OP>>(m.nslices, st, sell_of<S>(m), x, b,
                                                     a, status);
       return;
     }
   }
   if (m.sell) {
-    launch_body<sell_start_kernel<S, V, RB, CB, OP>>(sell_grid(m.nslices), sell_threads(), 0, st, sell_of<S>(m), x, b,
+    launch_walk<sell_start_kernel<S, V, RB, CB, OP>>(m.nslices, st, sell_of<S>(m), x, b,
                                                      a, status);
     return;
   }
