@@ -741,19 +741,72 @@ __global__ void nodal_field_kernel(const double* __restrict__ nodes, const uint3
   vm[n] = sqrt(0.5 * (a0 * a0 + b0 * b0 + c0 * c0) + 3.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]));
 }
 
-__global__ void scatter_displacements_kernel(const double* __restrict__ x, const uint32_t* __restrict__ free,
-                                             uint32_t count, double* __restrict__ disp) {
-  uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= count) return;
-  uint32_t f = free[n];
-  for (int k = 0; k < 3; ++k) disp[(size_t)n * 3 + k] = f == 0xffffffffu ? 0.0 : x[(size_t)f * 3 + k];
+// disp (zeros) at every free row's node from the free-DOF solution.
+__global__ void scatter_displacements_kernel(const double* __restrict__ x, const uint32_t* __restrict__ row_node,
+                                             size_t count, double* __restrict__ disp) {
+  const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (i < count) disp[(size_t)row_node[i / 3] * 3 + i % 3] = x[i];
+}
+
+// The recovery's incidence (results.rs:414-435) from the assembly's: each node's (element, local
+// node) in element order, and each midside node's first element and edge slot. A vertex's elements
+// are its node's elements as they stand (a vertex is only ever a corner).
+__global__ void node_incidence_kernel(const uint32_t* __restrict__ tets, uint32_t nodes, uint32_t vertices,
+                                      const uint32_t* __restrict__ inc_start, const uint32_t* __restrict__ inc,
+                                      uint32_t* __restrict__ node_incident, uint32_t* __restrict__ midside_first) {
+  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  if (n >= nodes) return;
+  for (uint32_t k = inc_start[n]; k < inc_start[n + 1]; ++k) {
+    const uint32_t e = inc[k];
+    uint32_t a = 0;
+    while (a < 9 && tets[(size_t)e * 10 + a] != n) ++a;
+    node_incident[k] = (e << 4) | a;
+    if (n >= vertices && k == inc_start[n]) midside_first[n - vertices] = (e << 3) | (a - 4);
+  }
+}
+
+// Points [first, first + count) as the API's records (sf_point_stress: 22 words each), a thread per
+// word, so a warp writes 128 consecutive bytes.
+__global__ void pack_points_kernel(const double* __restrict__ stress, const double* __restrict__ vm,
+                                   const double* __restrict__ pos, uint32_t points, size_t first, size_t count,
+                                   uint32_t* __restrict__ out) {
+  const size_t w = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (w >= count * 22) return;
+  const size_t i = first + w / 22;
+  const uint32_t f = (uint32_t)(w % 22);
+  uint32_t v;
+  if (f == 0) v = (uint32_t)(i / points);
+  else if (f == 1) v = (uint32_t)(i % points);
+  else if (f < 8) v = reinterpret_cast<const uint32_t*>(pos)[i * 6 + f - 2];
+  else if (f < 20) v = reinterpret_cast<const uint32_t*>(stress)[i * 12 + f - 8];
+  else v = reinterpret_cast<const uint32_t*>(vm)[i * 2 + f - 20];
+  out[w] = v;
 }
 
 }  // namespace
 
-sf_status launch_scatter_displacements(const double* x, RecoveryDevice& r, uint32_t node_count, cudaStream_t stream) {
-  scatter_displacements_kernel<<<(node_count + 255) / 256, 256, 0, stream>>>(x, r.free, node_count, r.disp);
+sf_status launch_scatter_displacements(const double* x, const uint32_t* row_node, size_t rows, double* disp,
+                                       cudaStream_t stream) {
+  if (rows == 0) return SF_OK;
+  scatter_displacements_kernel<<<(unsigned)((3 * rows + 255) / 256), 256, 0, stream>>>(x, row_node, 3 * rows, disp);
   return cuda_check(cudaGetLastError(), "scatter displacements");
+}
+
+sf_status launch_node_incidence(const AssemblyDevice& a, uint32_t node_count, uint32_t vertex_count, uint32_t* incident,
+                                uint32_t* midside_first, cudaStream_t stream) {
+  node_incidence_kernel<<<(node_count + 127) / 128, 128, 0, stream>>>(a.tets, node_count, vertex_count, a.inc_start,
+                                                                      a.inc, incident, midside_first);
+  return cuda_check(cudaGetLastError(), "recovery incidence");
+}
+
+sf_status launch_pack_points(const RecoveryDevice& r, int points, size_t first, size_t count, void* out,
+                             cudaStream_t stream) {
+  static_assert(sizeof(sf_point_stress) == 88, "a point record is 22 words");
+  if (count == 0) return SF_OK;
+  pack_points_kernel<<<(unsigned)((count * 22 + 255) / 256), 256, 0, stream>>>(r.point_stress, r.point_vm, r.point_pos,
+                                                                               (uint32_t)points, first, count,
+                                                                               (uint32_t*)out);
+  return cuda_check(cudaGetLastError(), "pack points");
 }
 
 sf_status launch_recovery_elements(const AssemblyDevice& a, const MaterialSpec& m, RecoveryDevice& r, uint32_t first,

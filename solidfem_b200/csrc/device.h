@@ -301,22 +301,21 @@ sf_status launch_gather(const AssemblyDevice& a, DevBsr& system, uint32_t end, c
 // values and patch fits, then the nodal field.
 struct RecoveryDevice {
   double* disp = nullptr;         // node_count x 3
-  uint32_t* free = nullptr;       // node_count: free index or FIXED
   double* point_stress = nullptr; // tet_count x points x 6
   double* point_vm = nullptr;     // tet_count x points
   double* point_pos = nullptr;    // tet_count x points x 3
   double* point_mat = nullptr;    // tet_count x points x 2
   double* node_candidate = nullptr;  // tet_count x 10 x 7: stress and von Mises at each node
-  uint32_t* vertex_offsets = nullptr;  // vertex_count + 1
-  uint32_t* vertex_incident = nullptr; // elements touching each vertex, ascending
-  uint32_t* node_offsets = nullptr;    // node_count + 1: (element, local node) incidence
+  const uint32_t* vertex_offsets = nullptr;  // vertex_count + 1 (the assembly's incidence)
+  const uint32_t* vertex_incident = nullptr; // elements touching each vertex, ascending
+  const uint32_t* node_offsets = nullptr;    // node_count + 1: (element, local node) incidence
   uint32_t* node_incident = nullptr;   // (element << 4) | local node, ascending element
   double* fits = nullptr;         // vertex_count x 28: centre (3), scale, coefficients (4 x 6)
   int* has_fit = nullptr;         // vertex_count
   uint32_t* midside_first = nullptr;  // per midside node: (first element << 3) | edge slot
   double* nodal_stress = nullptr; // node_count x 6
   double* nodal_vm = nullptr;     // node_count
-  bool ready = false;             // incidence uploaded
+  bool ready = false;             // incidence made
 };
 // Device stress recovery of the displacements in r.disp (crates/solidfem-elastic/src/results.rs:
 // 470-539 and 376-410, patch.rs:37-120), bit-identical to the reference's serial recovery, in
@@ -329,8 +328,16 @@ sf_status launch_recovery_fits(const AssemblyDevice& a, RecoveryDevice& r, uint3
                                cudaStream_t stream);
 sf_status launch_recovery_field(const AssemblyDevice& a, RecoveryDevice& r, uint32_t node_count,
                                 uint32_t vertex_count, cudaStream_t stream);
-// The displacement of every mesh node from the free-DOF solution (zero at fixed nodes).
-sf_status launch_scatter_displacements(const double* x, RecoveryDevice& r, uint32_t node_count, cudaStream_t stream);
+// The displacement of every free row's node from the free-DOF solution, into zeros.
+sf_status launch_scatter_displacements(const double* x, const uint32_t* row_node, size_t rows, double* disp,
+                                       cudaStream_t stream);
+// The recovery's per-node (element << 4 | local node) list, laid out as a.inc, and its midsides'
+// first elements, from the assembly's incidence.
+sf_status launch_node_incidence(const AssemblyDevice& a, uint32_t node_count, uint32_t vertex_count, uint32_t* incident,
+                                uint32_t* midside_first, cudaStream_t stream);
+// Points [first, first + count) as sf_point_stress records.
+sf_status launch_pack_points(const RecoveryDevice& r, int points, size_t first, size_t count, void* out,
+                             cudaStream_t stream);
 
 // ------------------------------------------------------------------- solve (solve.cu)
 // Uploads the hierarchy in the study's precision and allocates every work vector.

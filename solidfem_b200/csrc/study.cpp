@@ -462,6 +462,104 @@ extern "C" {
 static void recovery_free(sf_recovery* r);  // defined with the recovery entry points
 }
 
+// ------------------------------------------------------------ large arrays over the host link
+// An array of megabytes crosses in chunks through two pooled pinned buffers, so that the link moves
+// one chunk at its own rate while `threads` host threads copy the other; a copy to or from pageable
+// memory runs on one thread in the driver, page faults of a fresh result array included (the gate
+// plate's 57 MB of fields, with the point records put together on the device instead of the host:
+// 20.6 -> 3.8 ms a call; the 60^3 block's 42 MB of displacements 23 -> 4 ms).
+namespace {
+
+constexpr size_t kCopyChunk = (size_t)4 << 20;
+constexpr size_t kSmallCopy = (size_t)64 << 10;       // below this the driver's own staging is as quick
+constexpr size_t kDeviceFieldNodes = 16384;           // fields of fewer nodes are spread on the host
+
+int host_threads(const sf_study* s) {
+  return s->options.threads ? (int)std::min<uint64_t>(s->options.threads, 64) : default_threads();
+}
+
+void host_copy(void* dst, const void* src, size_t bytes, int threads) {
+  const int parts = bytes < ((size_t)1 << 20) ? 1 : threads;
+#ifdef _OPENMP
+#pragma omp parallel for schedule(static, 1) num_threads(parts) if (parts > 1)
+#endif
+  for (int p = 0; p < parts; ++p) {
+    const size_t b = bytes * (size_t)p / parts / 64 * 64, e = p + 1 == parts ? bytes : bytes * (size_t)(p + 1) / parts / 64 * 64;
+    std::memcpy((char*)dst + b, (const char*)src + b, e - b);
+  }
+}
+
+// Two pinned chunks and their events; the buffers go back to the pool once nothing uses them.
+struct Staging {
+  void* buf[2] = {nullptr, nullptr};
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  bool ok = true;
+  explicit Staging(size_t chunk) {
+    for (int i = 0; i < 2; ++i) {
+      buf[i] = pinned_acquire(chunk);
+      ok = buf[i] && cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming) == cudaSuccess && ok;
+    }
+  }
+  ~Staging() {
+    for (int i = 0; i < 2; ++i) {
+      if (buf[i]) pinned_return(buf[i]);
+      if (done[i]) cudaEventDestroy(done[i]);
+    }
+  }
+};
+
+// Device bytes to host memory, complete on return. `from(at, len)` gives the device address of the
+// bytes [at, at + len) of a chunk, enqueueing what makes them on d.stream first.
+template <class F>
+sf_status copy_out(const DeviceSolver& d, void* dst, size_t bytes, size_t chunk, int threads, F&& from) {
+  if (bytes < kSmallCopy) {
+    if (bytes) copy_d2h(d, dst, from(0, bytes), bytes);
+    return cuda_check(cudaStreamSynchronize(d.stream), "copy to the host");
+  }
+  Staging st(std::min(chunk, bytes));
+  if (!st.ok) return fail(SF_CUDA_ERROR, "cudaMallocHost failed");
+  const size_t count = (bytes + chunk - 1) / chunk;
+  sf_status e = SF_OK;
+  for (size_t i = 0; i <= count && !e; ++i) {
+    if (i < count) {
+      const size_t at = i * chunk, len = std::min(chunk, bytes - at);
+      copy_d2h(d, st.buf[i & 1], from(at, len), len);
+      cudaEventRecord(st.done[i & 1], d.stream);
+    }
+    if (i > 0) {
+      const size_t at = (i - 1) * chunk, len = std::min(chunk, bytes - at);
+      e = cuda_check(cudaEventSynchronize(st.done[(i - 1) & 1]), "copy to the host");
+      if (!e) host_copy((char*)dst + at, st.buf[(i - 1) & 1], len, threads);
+    }
+  }
+  const sf_status end = cuda_check(cudaStreamSynchronize(d.stream), "copy to the host");
+  return e ? e : end;
+}
+
+// Host bytes to device memory (and to `keep`, when given), complete on return.
+sf_status copy_in(const DeviceSolver& d, void* dst, const void* src, void* keep, size_t bytes, int threads) {
+  if (bytes < kSmallCopy) {
+    if (keep) std::memcpy(keep, src, bytes);
+    if (bytes) copy_h2d(d, dst, src, bytes);
+    return SF_OK;
+  }
+  Staging st(std::min(kCopyChunk, bytes));
+  if (!st.ok) return fail(SF_CUDA_ERROR, "cudaMallocHost failed");
+  sf_status e = SF_OK;
+  for (size_t i = 0, at = 0; at < bytes && !e; ++i, at += kCopyChunk) {
+    const size_t len = std::min(kCopyChunk, bytes - at);
+    if (i >= 2) e = cuda_check(cudaEventSynchronize(st.done[i & 1]), "copy to the device");
+    host_copy(st.buf[i & 1], (const char*)src + at, len, threads);
+    copy_h2d(d, (char*)dst + at, st.buf[i & 1], len);
+    cudaEventRecord(st.done[i & 1], d.stream);
+    if (keep) host_copy((char*)keep + at, (const char*)src + at, len, threads);
+  }
+  const sf_status end = cuda_check(cudaStreamSynchronize(d.stream), "copy to the device");
+  return e ? e : end;
+}
+
+}  // namespace
+
 void sf_study::release_answer() {
   if (answer) recovery_free(answer);
   answer = nullptr;
@@ -1106,11 +1204,12 @@ static sf_status builder_assemble(sf_builder* b, uint64_t max_elements, sf_cance
         return me;
       }
     }
-    // The element stiffness buffer and the assembly map have served; free them for the solve.
-    for (void* p : {(void*)a.ke, (void*)a.inc_start, (void*)a.inc, (void*)a.row_node, (void*)a.cursor})
-      dev_free(s, p);
+    // The element stiffness buffer and the rows' cursors have served; free them for the solve. The
+    // incidence and the rows' nodes stay for the recovery and the displacements.
+    dev_free(s, a.ke);
+    dev_free(s, a.cursor);
     a.ke = nullptr;
-    a.inc_start = a.inc = a.row_node = a.cursor = nullptr;
+    a.cursor = nullptr;
   }
   return SF_OK;
 }
@@ -1559,12 +1658,29 @@ sf_status sf_study_solve_batch(sf_study** studies, uint64_t count, sf_step_outco
 sf_status sf_study_displacements(const sf_study* s, double* out) {
   if (!s || !out) return fail(SF_INVALID_ARGUMENT, "null argument");
   const DeviceSolver& d = s->solver;
-  vector<double> x(d.n);
   cudaSetDevice(d.device);
-  copy_d2h(d, x.data(), d.x, (size_t)d.n * 8);
-  if (sf_status e = cuda_check(cudaStreamSynchronize(d.stream), "read displacements")) return e;
-  for (size_t n = 0; n < s->free.size(); ++n)
-    for (int a = 0; a < 3; ++a) out[3 * n + a] = s->free[n] == FIXED ? 0.0 : x[3 * (size_t)s->free[n] + a];
+  const size_t nn = s->free.size();
+  // Large fields are spread over the nodes on the device and come to the caller's memory through
+  // pinned buffers; small ones, or when the device has no room for one, are spread here.
+  double* field = nullptr;
+  pool_setup(d.device);
+  if (nn >= kDeviceFieldNodes && cudaMallocAsync((void**)&field, nn * 24, d.stream) != cudaSuccess) {
+    cudaGetLastError();
+    field = nullptr;
+  }
+  if (field) {
+    cudaMemsetAsync(field, 0, nn * 24, d.stream);
+    sf_status e = launch_scatter_displacements(d.x, s->asmdev.row_node, s->free_count, field, d.stream);
+    if (!e) e = copy_out(d, out, nn * 24, kCopyChunk, host_threads(s), [&](size_t at, size_t) { return (char*)field + at; });
+    cudaFreeAsync(field, d.stream);
+    if (e) return e;
+  } else {
+    vector<double> x(d.n);
+    copy_d2h(d, x.data(), d.x, (size_t)d.n * 8);
+    if (sf_status e = cuda_check(cudaStreamSynchronize(d.stream), "read displacements")) return e;
+    for (size_t n = 0; n < nn; ++n)
+      for (int a = 0; a < 3; ++a) out[3 * n + a] = s->free[n] == FIXED ? 0.0 : x[3 * (size_t)s->free[n] + a];
+  }
   // A prescribed component is exact, not the solver's estimate of it (study.rs:233-236).
   for (auto& p : s->model.prescribed) out[3 * (size_t)p.first.first + p.first.second] = p.second;
   return SF_OK;
@@ -1577,7 +1693,7 @@ sf_status sf_study_report(const sf_study* s, sf_report* out) {
 }
 
 // Device stress recovery (Recovery, results.rs:97-124, 376-539). The incidence lists every
-// recovery of a study reads are built once on the host; a recovery snapshots the displacements on
+// recovery of a study reads are made once, from the assembly's; a recovery snapshots the displacements on
 // the device and advances in the reference's units of work (each element, then each vertex's
 // patch fit); the nodal field is made when both are done.
 static sf_status recovery_tables(sf_study* s) {
@@ -1585,41 +1701,15 @@ static sf_status recovery_tables(sf_study* s) {
   if (r.ready) return SF_OK;
   DeviceSolver& d = s->solver;
   const Mesh& m = s->model.mesh;
-  const size_t nn = m.nodes.size(), ne = m.tets.size(), nv = m.vertex_count;
-  // Elements touching each vertex through a corner, and (element, local node) per node, both in
-  // element order (results.rs:414-435); the first element reaching each midside node.
-  vector<uint32_t> voff(nv + 1, 0), noff(nn + 1, 0);
-  for (auto& t : m.tets) {
-    for (int c = 0; c < 4; ++c) voff[t[c] + 1] += 1;
-    for (int a = 0; a < 10; ++a) noff[t[a] + 1] += 1;
-  }
-  for (size_t i = 0; i < nv; ++i) voff[i + 1] += voff[i];
-  for (size_t i = 0; i < nn; ++i) noff[i + 1] += noff[i];
-  vector<uint32_t> vinc(voff[nv]), ninc(noff[nn]);
-  vector<uint32_t> vf(voff.begin(), voff.end() - 1), nf(noff.begin(), noff.end() - 1);
-  vector<uint32_t> mid(nn - nv, 0xffffffffu);
-  for (size_t e = 0; e < ne; ++e) {
-    const auto& t = m.tets[e];
-    for (int c = 0; c < 4; ++c) vinc[vf[t[c]]++] = (uint32_t)e;
-    for (int a = 0; a < 10; ++a) ninc[nf[t[a]]++] = ((uint32_t)e << 4) | (uint32_t)a;
-    for (int k = 0; k < 6; ++k)
-      if (mid[t[4 + k] - nv] == 0xffffffffu) mid[t[4 + k] - nv] = ((uint32_t)e << 3) | (uint32_t)k;
-  }
-  sf_status e = SF_OK;
-  if (!e) e = dev_alloc(d, (void**)&r.free, nn * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.vertex_offsets, (nv + 1) * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.vertex_incident, std::max<size_t>(1, vinc.size()) * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.node_offsets, (nn + 1) * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.node_incident, std::max<size_t>(1, ninc.size()) * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.midside_first, std::max<size_t>(1, mid.size()) * 4);
+  const size_t nn = m.nodes.size(), nv = m.vertex_count;
+  sf_status e = dev_alloc(d, (void**)&r.node_incident, std::max<size_t>(1, 10 * m.tets.size()) * 4);
+  if (!e) e = dev_alloc(d, (void**)&r.midside_first, std::max<size_t>(1, nn - nv) * 4);
   if (e) return e;
-  copy_h2d(d, r.free, s->free.data(), nn * 4);
-  copy_h2d(d, r.vertex_offsets, voff.data(), voff.size() * 4);
-  if (!vinc.empty()) copy_h2d(d, r.vertex_incident, vinc.data(), vinc.size() * 4);
-  copy_h2d(d, r.node_offsets, noff.data(), noff.size() * 4);
-  if (!ninc.empty()) copy_h2d(d, r.node_incident, ninc.data(), ninc.size() * 4);
-  if (!mid.empty()) copy_h2d(d, r.midside_first, mid.data(), mid.size() * 4);
-  if ((e = cuda_check(cudaStreamSynchronize(d.stream), "recovery set-up"))) return e;
+  r.vertex_offsets = r.node_offsets = s->asmdev.inc_start;
+  r.vertex_incident = s->asmdev.inc;
+  if ((e = launch_node_incidence(s->asmdev, (uint32_t)nn, (uint32_t)nv, r.node_incident, r.midside_first, d.stream)))
+    return e;
+  d.launches += 1;
   r.ready = true;
   return SF_OK;
 }
@@ -1665,7 +1755,7 @@ static sf_status recovery_begin(sf_study* s, sf_recovery** out) {
   if (!e) e = alloc((void**)&r.has_fit, nv * 4);
   if (!e) e = alloc((void**)&r.nodal_stress, nn * 48);
   if (!e) e = alloc((void**)&r.nodal_vm, nn * 8);
-  if (!e) e = launch_scatter_displacements(d.x, r, (uint32_t)nn, d.stream);
+  if (!e) e = launch_scatter_displacements(d.x, s->asmdev.row_node, s->free_count, r.disp, d.stream);
   if (!e && !s->model.prescribed.empty()) {
     // the prescribed components, exact
     vector<uint32_t> idx;
@@ -1751,28 +1841,32 @@ static sf_status recovery_outputs(sf_study* s, sf_recovery* rec, double* displac
   sf_status e = launch_recovery_field(s->asmdev, rec->dev, (uint32_t)nn, (uint32_t)m.vertex_count, d.stream);
   d.launches += 1;
   if (e) return e;
-  if (displacements) copy_d2h(d, displacements, rec->dev.disp, nn * 24);
-  if (nodal_stress) copy_d2h(d, nodal_stress, rec->dev.nodal_stress, nn * 48);
-  if (nodal_von_mises) copy_d2h(d, nodal_von_mises, rec->dev.nodal_vm, nn * 8);
-  vector<double> ps, pv, pp;
-  if (points) {
-    ps.resize(pts * 6);
-    pv.resize(pts);
-    pp.resize(pts * 3);
-    copy_d2h(d, ps.data(), rec->dev.point_stress, pts * 48);
-    copy_d2h(d, pv.data(), rec->dev.point_vm, pts * 8);
-    copy_d2h(d, pp.data(), rec->dev.point_pos, pts * 24);
-  }
-  if ((e = cuda_check(cudaStreamSynchronize(d.stream), "read recovery"))) return e;
-  if (points)
-    for (size_t i = 0; i < pts; ++i) {
-      points[i].tet = (uint32_t)(i / q);
-      points[i].point = (uint32_t)(i % q);
-      for (int k = 0; k < 3; ++k) points[i].position[k] = pp[i * 3 + k];
-      for (int k = 0; k < 6; ++k) points[i].stress[k] = ps[i * 6 + k];
-      points[i].von_mises = pv[i];
-    }
-  return SF_OK;
+  const int threads = host_threads(s);
+  auto plain = [&](void* dst, const void* dev, size_t bytes) {
+    return dst ? copy_out(d, dst, bytes, kCopyChunk, threads, [&](size_t at, size_t) { return (const char*)dev + at; })
+               : SF_OK;
+  };
+  e = plain(displacements, rec->dev.disp, nn * 24);
+  if (!e) e = plain(nodal_stress, rec->dev.nodal_stress, nn * 48);
+  if (!e) e = plain(nodal_von_mises, rec->dev.nodal_vm, nn * 8);
+  if (!points || e) return e;
+  // The point records are put together on the device, a chunk at a time in two small buffers.
+  constexpr size_t kRecords = kCopyChunk / sizeof(sf_point_stress), kBytes = kRecords * sizeof(sf_point_stress);
+  void* packed[2] = {nullptr, nullptr};
+  const size_t each = std::min(kBytes, pts * sizeof(sf_point_stress));
+  for (void*& p : packed)
+    if (!e) e = dev_alloc(d, &p, std::max<size_t>(each, 8));
+  sf_status pe = SF_OK;
+  int turn = 0;
+  if (!e)
+    e = copy_out(d, points, pts * sizeof(sf_point_stress), kBytes, threads, [&](size_t at, size_t len) {
+      void* p = packed[turn ^= 1];
+      if (!pe) pe = launch_pack_points(rec->dev, (int)q, at / sizeof(sf_point_stress), len / sizeof(sf_point_stress), p, d.stream);
+      d.launches += 1;
+      return p;
+    });
+  for (void* p : packed) dev_free(d, p);
+  return e ? e : pe;
 }
 
 // Units of recovery work per launch when the caller gives no budget (sf_study_solution): the
@@ -2059,10 +2153,8 @@ sf_status sf_study_resolve(sf_study* s, const double* rhs) {
   if (!s) return fail(SF_INVALID_ARGUMENT, "null argument");
   DeviceSolver& d = s->solver;
   cudaSetDevice(d.device);
-  if (rhs) {
-    std::memcpy(s->rhs.data(), rhs, (size_t)d.n * 8);
-    copy_h2d(d, d.rhs, rhs, (size_t)d.n * 8);
-  }
+  if (rhs)
+    if (sf_status e = copy_in(d, d.rhs, rhs, s->rhs.data(), (size_t)d.n * 8, host_threads(s))) return e;
   if (sf_status e = solver_restart(d, s->options.tolerance, s->options.max_iterations)) return e;
   s->release_answer();
   s->cancelled = false;
