@@ -98,6 +98,14 @@ struct PcgState {
   unsigned int tickets[8];
 };
 
+// Iterations in the longer graph of a small solver. Between two graphs the last kernel must finish
+// and the next graph start, 6 us in which nothing runs, where kernels of one graph follow each other
+// by programmatic launches: 69.8 -> 64.0 us an iteration at 9,720 unknowns, no difference at 217,800
+// (345 us an iteration). Its capture costs as much as a few dozen of those gaps, so it is made once a
+// solver has run kRunAfter iterations.
+static const uint64_t kRunIterations = 4;
+static const uint64_t kRunAfter = 64;
+static const uint32_t kRunMaxUnknowns = 151552;
 // Reduction scratch: one partial per block of the fixed reduction grid.
 static const int kReduceBlocks = 592;  // 4 x 148 SMs
 static const int kReduceThreads = 256;
@@ -139,6 +147,9 @@ struct DeviceSolver {
   size_t bytes = 0;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
+  cudaGraph_t run_graph = nullptr;           // kRunIterations iterations in one graph
+  cudaGraphExec_t run_exec = nullptr;
+  uint64_t iterations_run = 0;               // by this solver, over all its solves
   uint64_t launches_per_iteration = 0;
   uint64_t graph_kernels = 0;     // kernel nodes in the captured iteration graph
   uint64_t launches = 0;          // kernels launched so far (graph replays count their kernels)
@@ -219,6 +230,11 @@ sf_status setup_strength(cudaStream_t st, uint32_t rows, const uint32_t* starts,
 sf_status setup_union_rows(cudaStream_t st, uint32_t rows, uint32_t width, const uint32_t* outer_starts,
                            const uint32_t* outer_idx, bool self, const uint32_t* inner_starts,
                            const uint32_t* inner_cols, const uint32_t* out_starts, uint32_t* out);
+// The 3x3 blocks of a scalar CSR matrix of n rows (columns ascending) over `rows` = ceil(n / 3) block
+// rows, the padding rows' diagonal included: out_starts null counts each block row's blocks into
+// out; else the block columns go to out[out_starts[row] ..] and the entries into vals (zeros before).
+sf_status setup_padded_blocks(cudaStream_t st, uint64_t n, uint32_t rows, const uint64_t* rs, const uint32_t* cols,
+                              const double* scalars, const uint32_t* out_starts, uint32_t* out, double* vals);
 // Listed blocks of len values out of / back into a block array; out[idx[i]] = vals[i].
 sf_status setup_gather_blocks(cudaStream_t st, size_t count, int len, const uint32_t* idx, const double* in,
                               double* out);
@@ -355,6 +371,7 @@ sf_status solver_level_stage(DeviceSolver& s, size_t level, int stage, const dou
 sf_status solver_precondition(DeviceSolver& s, const double* d_in, double* d_out);
 sf_status solver_system_multiply(DeviceSolver& s, const double* d_in, double* d_out);
 sf_status solver_capture_graph(DeviceSolver& s);
+sf_status solver_capture_run(DeviceSolver& s);  // kRunIterations iterations
 sf_status solver_read_state(DeviceSolver& s, PcgState* out);
 // Pcg::step on the device (study.cpp): up to max_iterations iterations replayed in chunks with one
 // state read-back per chunk into `pinned`; updates last, status and cancelled.

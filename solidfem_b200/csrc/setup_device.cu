@@ -877,6 +877,44 @@ __global__ void split_fill_kernel(size_t slots, const uint32_t* __restrict__ sel
   }
 }
 
+// A thread per block row merges its three scalar rows: the next block column is the least of the
+// rows' next columns over three (and, for the padded last block row, its own diagonal block).
+__global__ void padded_blocks_kernel(uint64_t n, uint32_t rows, const uint64_t* __restrict__ rs,
+                                     const uint32_t* __restrict__ cols, const double* __restrict__ scalars,
+                                     const uint32_t* __restrict__ out_starts, uint32_t* __restrict__ out,
+                                     double* __restrict__ vals) {
+  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= rows) return;
+  uint64_t at[3], end[3];
+  for (int p = 0; p < 3; ++p) {
+    const uint64_t r = 3 * (uint64_t)b + p;
+    at[p] = r < n ? rs[r] : 0;
+    end[p] = r < n ? rs[r + 1] : 0;
+  }
+  bool own = 3 * (uint64_t)b + 3 > n;  // the padding's diagonal block is still to come
+  uint32_t count = 0;
+  const size_t first = out_starts ? out_starts[b] : 0;
+  for (;;) {
+    uint32_t c = own ? b : 0xffffffffu;
+    for (int p = 0; p < 3; ++p)
+      if (at[p] < end[p]) c = min(c, cols[at[p]] / 3);
+    if (c == 0xffffffffu) break;
+    if (c == b) own = false;
+    double* v = vals + (first + count) * 9;
+    for (int p = 0; p < 3; ++p)
+      for (; at[p] < end[p] && cols[at[p]] / 3 == c; ++at[p])
+        if (out_starts) v[3 * p + cols[at[p]] % 3] = scalars[at[p]];
+    if (out_starts) {
+      out[first + count] = c;
+      if (c == b)
+        for (int p = 0; p < 3; ++p)
+          if (3 * (uint64_t)b + p >= n) v[4 * p] = 1.0;
+    }
+    ++count;
+  }
+  if (!out_starts) out[b] = count;
+}
+
 // Copies listed blocks out of (gather) or back into (scatter) a block array.
 __global__ void gather_blocks_kernel(size_t count, int len, const uint32_t* __restrict__ idx,
                                      const double* __restrict__ in, double* __restrict__ out) {
@@ -895,6 +933,13 @@ __global__ void set_values_kernel(size_t count, const uint32_t* __restrict__ idx
 }
 
 }  // namespace
+
+sf_status setup_padded_blocks(cudaStream_t st, uint64_t n, uint32_t rows, const uint64_t* rs, const uint32_t* cols,
+                              const double* scalars, const uint32_t* out_starts, uint32_t* out, double* vals) {
+  if (rows == 0) return SF_OK;
+  padded_blocks_kernel<<<(rows + 127) / 128, 128, 0, st>>>(n, rows, rs, cols, scalars, out_starts, out, vals);
+  return cuda_check(cudaGetLastError(), "padded blocks");
+}
 
 sf_status setup_gather_blocks(cudaStream_t st, size_t count, int len, const uint32_t* idx, const double* in,
                               double* out) {

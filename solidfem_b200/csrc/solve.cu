@@ -178,8 +178,10 @@ void dev_free(DeviceSolver& s, void* ptr) {
 void dev_free_all(DeviceSolver& s) {
   if (s.graph_exec) cudaGraphExecDestroy(s.graph_exec);
   if (s.graph) cudaGraphDestroy(s.graph);
-  s.graph_exec = nullptr;
-  s.graph = nullptr;
+  if (s.run_exec) cudaGraphExecDestroy(s.run_exec);
+  if (s.run_graph) cudaGraphDestroy(s.run_graph);
+  s.graph_exec = s.run_exec = nullptr;
+  s.graph = s.run_graph = nullptr;
   for (auto& p : s.owned) cudaFreeAsync(p.first, s.stream);
   s.owned.clear();
   s.bytes = 0;
@@ -516,14 +518,20 @@ sf_status solver_init_pcg(DeviceSolver& s, double tolerance, uint64_t max_iterat
 }
 
 sf_status solver_enqueue_reset(DeviceSolver& s) {
-  const int* status = &s.state->status;
-  enqueue_precondition(s, s.r, s.z, s.z32, status);
-  if (s.vector_single && s.multigrid) {
-    launch_body<pcg_dot_rz_kernel<float>>(grid_for_reduction(s.n), kReduceThreads, 0, s.stream, s.n, s.r, s.z32, s.ap, s.partials, s.state);
-    launch_body<pcg_update_p_kernel<float>>(grid_for_elems(s.n), kThreads, 0, s.stream, s.n, s.z32, s.p, s.state);
+  const int grid = grid_for_reduction(s.n), wide = grid_for_elems(s.n);
+  if (!s.multigrid) {
+    // Jacobi: z = r / diag is formed where it is read, in both kernels.
+    launch_body<jacobi_dot_rz_kernel>(grid, kReduceThreads, 0, s.stream, s.n, s.r, s.jacobi, s.ap, s.partials, s.state);
+    launch_body<jacobi_update_p_kernel>(wide, kThreads, 0, s.stream, s.n, s.r, s.jacobi, s.p, s.state);
   } else {
-    launch_body<pcg_dot_rz_kernel<double>>(grid_for_reduction(s.n), kReduceThreads, 0, s.stream, s.n, s.r, s.z, s.ap, s.partials, s.state);
-    launch_body<pcg_update_p_kernel<double>>(grid_for_elems(s.n), kThreads, 0, s.stream, s.n, s.z, s.p, s.state);
+    enqueue_precondition(s, s.r, s.z, s.z32, &s.state->status);
+    if (s.vector_single) {
+      launch_body<pcg_dot_rz_kernel<float>>(grid, kReduceThreads, 0, s.stream, s.n, s.r, s.z32, s.ap, s.partials, s.state);
+      launch_body<pcg_update_p_kernel<float>>(wide, kThreads, 0, s.stream, s.n, s.z32, s.p, s.state);
+    } else {
+      launch_body<pcg_dot_rz_kernel<double>>(grid, kReduceThreads, 0, s.stream, s.n, s.r, s.z, s.ap, s.partials, s.state);
+      launch_body<pcg_update_p_kernel<double>>(wide, kThreads, 0, s.stream, s.n, s.z, s.p, s.state);
+    }
   }
   s.launches_per_iteration += 2;
   return cuda_check(cudaGetLastError(), "reset direction");
@@ -531,7 +539,6 @@ sf_status solver_enqueue_reset(DeviceSolver& s) {
 
 sf_status solver_enqueue_iteration(DeviceSolver& s) {
   cudaStream_t st = s.stream;
-  const int* status = &s.state->status;
   s.launches_per_iteration = 0;
   if (s.system.sell) {
     SellOp<double> A = sell_of<double>(s.system);
@@ -545,33 +552,36 @@ sf_status solver_enqueue_iteration(DeviceSolver& s) {
     default: launch_pcg_spmv_lpr<32>(s); break;
   }
   s.launches_per_iteration += 3;
-  enqueue_precondition(s, s.r, s.z, s.z32, status);
-  if (s.vector_single && s.multigrid) {
-    launch_body<pcg_dot_rz_kernel<float>>(grid_for_reduction(s.n), kReduceThreads, 0, st, s.n, s.r, s.z32, s.ap, s.partials, s.state);
-    launch_body<pcg_update_p_kernel<float>>(grid_for_elems(s.n), kThreads, 0, st, s.n, s.z32, s.p, s.state);
-  } else {
-    launch_body<pcg_dot_rz_kernel<double>>(grid_for_reduction(s.n), kReduceThreads, 0, st, s.n, s.r, s.z, s.ap, s.partials, s.state);
-    launch_body<pcg_update_p_kernel<double>>(grid_for_elems(s.n), kThreads, 0, st, s.n, s.z, s.p, s.state);
-  }
-  s.launches_per_iteration += 2;
-  return cuda_check(cudaGetLastError(), "iteration");
+  return solver_enqueue_reset(s);
 }
+
+namespace {
+sf_status capture_iterations(DeviceSolver& s, uint64_t count, cudaGraph_t* graph, cudaGraphExec_t* exec) {
+  cudaError_t e = cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return cuda_check(e, "begin capture");
+  sf_status st = SF_OK;
+  for (uint64_t i = 0; i < count && !st; ++i) st = solver_enqueue_iteration(s);
+  cudaGraph_t g = nullptr;
+  e = cudaStreamEndCapture(s.stream, &g);
+  *graph = g;
+  if (st) return st;
+  if (e != cudaSuccess) return cuda_check(e, "end capture");
+  return cuda_check(cudaGraphInstantiate(exec, g, 0), "graph instantiate");
+}
+}  // namespace
 
 sf_status solver_capture_graph(DeviceSolver& s) {
   if (s.graph_exec) return SF_OK;
-  cudaError_t e = cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) return cuda_check(e, "begin capture");
-  sf_status st = solver_enqueue_iteration(s);
-  cudaGraph_t g = nullptr;
-  e = cudaStreamEndCapture(s.stream, &g);
-  if (st) return st;
-  if (e != cudaSuccess) return cuda_check(e, "end capture");
-  s.graph = g;
+  if (sf_status e = capture_iterations(s, 1, &s.graph, &s.graph_exec)) return e;
   size_t nodes = 0;
-  cudaGraphGetNodes(g, nullptr, &nodes);
+  cudaGraphGetNodes(s.graph, nullptr, &nodes);
   s.graph_kernels = nodes;
-  e = cudaGraphInstantiate(&s.graph_exec, g, 0);
-  return cuda_check(e, "graph instantiate");
+  return SF_OK;
+}
+
+sf_status solver_capture_run(DeviceSolver& s) {
+  if (s.run_exec) return SF_OK;
+  return capture_iterations(s, kRunIterations, &s.run_graph, &s.run_exec);
 }
 
 // ------------------------------------------------------------ batched iterations

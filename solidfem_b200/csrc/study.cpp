@@ -1427,7 +1427,16 @@ sf_status run_iterations(DeviceSolver& d, bool use_graphs, uint64_t max_iteratio
   while (!stop && done < max_iterations) {
     uint64_t k = std::min<uint64_t>(chunk, max_iterations - done);
     uint64_t launched = 0;
-    for (; launched < k; ++launched) {
+    while (launched < k) {
+      // Whole runs of iterations where no cancel must be read between them.
+      if (use_graphs && !cancel && k - launched >= kRunIterations && d.n <= kRunMaxUnknowns &&
+          d.iterations_run >= kRunAfter) {
+        if (sf_status e = solver_capture_run(d)) return e;
+        if (sf_status e = cuda_check(cudaGraphLaunch(d.run_exec, d.stream), "graph launch")) return e;
+        d.launches += kRunIterations * d.graph_kernels;
+        launched += kRunIterations;
+        continue;
+      }
       if (cancel && cancel(user)) {
         cancelled = true;
         stop = true;
@@ -1442,8 +1451,10 @@ sf_status run_iterations(DeviceSolver& d, bool use_graphs, uint64_t max_iteratio
         d.launches += d.launches_per_iteration;
       }
       if (e) return e;
+      ++launched;
     }
     done += launched;
+    d.iterations_run += launched;
     copy_d2h(d, pinned, d.state, sizeof(PcgState));
     if (sf_status e = cuda_check(cudaStreamSynchronize(d.stream), "solver step")) return e;
     last = *pinned;

@@ -108,46 +108,39 @@ sf_status from_nodal(uint64_t n, const uint64_t* rs, const uint32_t* cols, const
   return SF_OK;
 }
 
-// Any scalar matrix over ceil(n / 3) block rows: the blocks its entries touch (and the last
-// diagonal block when padding rows are added), zeros where it has no entry, identity on the
-// padding's diagonal.
-void padded_blocks(uint64_t n, const uint64_t* rs, const uint32_t* cols, const double* vals, vector<uint32_t>& starts,
-                   vector<uint32_t>& bcols, vector<double>& bvals) {
-  const uint64_t rows = (n + 2) / 3;
-  starts.assign(1, 0);
-  vector<uint32_t> mark(rows, UINT32_MAX);
-  vector<uint32_t> row_cols;
-  for (uint64_t b = 0; b < rows; ++b) {
-    row_cols.clear();
-    for (uint64_t r = 3 * b; r < std::min<uint64_t>(3 * b + 3, n); ++r)
-      for (uint64_t k = rs[r]; k < rs[r + 1]; ++k) {
-        uint32_t c = cols[k] / 3;
-        if (mark[c] != b) {
-          mark[c] = (uint32_t)b;
-          row_cols.push_back(c);
-        }
-      }
-    if (3 * b + 3 > n && mark[b] != b) row_cols.push_back((uint32_t)b);
-    std::sort(row_cols.begin(), row_cols.end());
-    const size_t first = bcols.size();
-    bcols.insert(bcols.end(), row_cols.begin(), row_cols.end());
-    bvals.resize(bcols.size() * 9, 0.0);
-    for (int p = 0; p < 3; ++p) {
-      const uint64_t r = 3 * b + p;
-      if (r >= n) {  // padding: a decoupled identity row
-        size_t at = std::lower_bound(bcols.begin() + first, bcols.end(), (uint32_t)b) - bcols.begin();
-        bvals[at * 9 + p * 3 + p] = 1.0;
-        continue;
-      }
-      size_t at = first;
-      for (uint64_t k = rs[r]; k < rs[r + 1]; ++k) {
-        const uint32_t c = cols[k] / 3;
-        while (bcols[at] != c) ++at;
-        bvals[at * 9 + p * 3 + cols[k] % 3] = vals[k];
-      }
-    }
-    starts.push_back((uint32_t)bcols.size());
+// Any scalar matrix over ceil(n / 3) block rows, on the device from its scalar rows: the blocks its
+// entries touch (and the last diagonal block when padding rows are added), zeros where it has no
+// entry, identity on the padding's diagonal. `starts` gets the block rows' starts.
+sf_status padded_blocks(DeviceSolver& d, uint64_t n, const uint64_t* rs, const uint32_t* cols, const double* vals,
+                        vector<uint32_t>& starts) {
+  const size_t rows = d.system.rows, entries = rs[n];
+  uint64_t* d_rs = nullptr;
+  uint32_t* d_cols = nullptr;
+  double* d_vals = nullptr;
+  sf_status e = dev_alloc(d, (void**)&d_rs, (n + 1) * 8);
+  if (!e) e = dev_alloc(d, (void**)&d_cols, std::max<size_t>(1, entries) * 4);
+  if (!e) e = dev_alloc(d, (void**)&d_vals, std::max<size_t>(1, entries) * 8);
+  if (e) return e;
+  copy_h2d(d, d_rs, rs, (n + 1) * 8);
+  if (entries) {
+    copy_h2d(d, d_cols, cols, entries * 4);
+    copy_h2d(d, d_vals, vals, entries * 8);
   }
+  e = setup_padded_blocks(d.stream, n, (uint32_t)rows, d_rs, d_cols, d_vals, nullptr, d.system.starts, nullptr);
+  starts.assign(rows + 1, 0);
+  if (!e) copy_d2h(d, starts.data() + 1, d.system.starts, rows * 4);
+  if (!e) e = cuda_check(cudaStreamSynchronize(d.stream), "system blocks");
+  if (e) return e;
+  for (size_t r = 0; r < rows; ++r) starts[r + 1] += starts[r];
+  const size_t blocks = d.system.blocks = starts[rows];
+  if (!e) e = dev_alloc(d, (void**)&d.system.cols, std::max<size_t>(1, blocks) * 4);
+  if (!e) e = dev_alloc(d, &d.system.vals, std::max<size_t>(1, blocks) * 72);  // zeros
+  if (e) return e;
+  copy_h2d(d, d.system.starts, starts.data(), (rows + 1) * 4);
+  e = setup_padded_blocks(d.stream, n, (uint32_t)rows, d_rs, d_cols, d_vals, d.system.starts, d.system.cols,
+                          (double*)d.system.vals);
+  for (void* p : {(void*)d_rs, (void*)d_cols, (void*)d_vals}) dev_free(d, p);
+  return e;
 }
 
 }  // namespace
@@ -173,7 +166,7 @@ sf_status sf_system_create(uint64_t n, const uint64_t* row_starts, const uint32_
   const sf_study_options& o = sys->options;
   const bool mg = o.preconditioner == SF_PRECONDITIONER_MULTIGRID;
   sys->n = n;
-  vector<double> bvals;
+  vector<double> bvals, diagonal;
   if (mg) {
     // MultigridSetup::new (setup.rs:129-160): the near-null length, the nodal blocks, then the
     // positions, each refused by name.
@@ -190,6 +183,7 @@ sf_status sf_system_create(uint64_t n, const uint64_t* row_starts, const uint32_
     }
   } else {
     // Jacobi::new (preconditioner.rs:49-79): a positive, finite diagonal.
+    diagonal.resize(n);
     for (uint64_t r = 0; r < n; ++r) {
       const uint32_t* lo = columns + row_starts[r];
       const uint32_t* hi = columns + row_starts[r + 1];
@@ -200,8 +194,8 @@ sf_status sf_system_create(uint64_t n, const uint64_t* row_starts, const uint32_
         error_slot().value = v;
         return fail(SF_JACOBI_DIAGONAL, "a diagonal entry is not positive");
       }
+      diagonal[r] = v;
     }
-    padded_blocks(n, row_starts, columns, values, sys->starts, sys->cols, bvals);
   }
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(SF_NO_DEVICE, "no CUDA device is visible");
@@ -212,20 +206,24 @@ sf_status sf_system_create(uint64_t n, const uint64_t* row_starts, const uint32_
   d.sell_min_rows = o.sell_min_rows ? o.sell_min_rows : 32768;
   d.coarse_tail = o.coarse_tail != 0;
   if (sf_status e = cuda_check(cudaStreamCreateWithFlags(&d.stream, cudaStreamNonBlocking), "stream")) return e;
-  const size_t rows = sys->starts.size() - 1, blocks = sys->cols.size();
+  const size_t rows = (n + 2) / 3;
   d.n = (uint32_t)(3 * rows);
   d.system.rows = (uint32_t)rows;
   d.system.rb = d.system.cb = 3;
-  d.system.blocks = blocks;
-  sf_status e = SF_OK;
-  if (!e) e = dev_alloc(d, (void**)&d.system.starts, (rows + 1) * 4);
-  if (!e) e = dev_alloc(d, (void**)&d.system.cols, std::max<size_t>(1, blocks) * 4);
-  if (!e) e = dev_alloc(d, &d.system.vals, std::max<size_t>(1, blocks) * 72);
+  sf_status e = dev_alloc(d, (void**)&d.system.starts, (rows + 1) * 4);
   if (e) return e;
-  copy_h2d(d, d.system.starts, sys->starts.data(), (rows + 1) * 4);
-  if (blocks) {
-    copy_h2d(d, d.system.cols, sys->cols.data(), blocks * 4);
-    copy_h2d(d, d.system.vals, bvals.data(), blocks * 72);
+  if (mg) {
+    const size_t blocks = d.system.blocks = sys->cols.size();
+    if (!e) e = dev_alloc(d, (void**)&d.system.cols, std::max<size_t>(1, blocks) * 4);
+    if (!e) e = dev_alloc(d, &d.system.vals, std::max<size_t>(1, blocks) * 72);
+    if (e) return e;
+    copy_h2d(d, d.system.starts, sys->starts.data(), (rows + 1) * 4);
+    if (blocks) {
+      copy_h2d(d, d.system.cols, sys->cols.data(), blocks * 4);
+      copy_h2d(d, d.system.vals, bvals.data(), blocks * 72);
+    }
+  } else if ((e = padded_blocks(d, n, row_starts, columns, values, sys->starts))) {
+    return e;
   }
   if ((e = make_row_groups(d, d.system, sys->starts.data(), 72))) return e;
   if ((e = cuda_check(cudaStreamSynchronize(d.stream), "system upload"))) return e;
@@ -262,12 +260,7 @@ sf_status sf_system_create(uint64_t n, const uint64_t* row_starts, const uint32_
     if (e) return e;
   } else {
     vector<double> inv(d.n, 1.0);
-    for (size_t b = 0; b < rows; ++b) {
-      const size_t at = std::lower_bound(sys->cols.begin() + sys->starts[b], sys->cols.begin() + sys->starts[b + 1],
-                                         (uint32_t)b) - sys->cols.begin();
-      for (int p = 0; p < 3; ++p)
-        if (3 * b + p < n) inv[3 * b + p] = 1.0 / bvals[at * 9 + p * 3 + p];
-    }
+    for (uint64_t r = 0; r < n; ++r) inv[r] = 1.0 / diagonal[r];
     if ((e = dev_alloc(d, (void**)&d.jacobi, (size_t)d.n * 8))) return e;
     copy_h2d(d, d.jacobi, inv.data(), (size_t)d.n * 8);
   }
