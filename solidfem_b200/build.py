@@ -24,7 +24,7 @@ CXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_COMMON = ["-O3", "-std=c++17", "-lineinfo", "-ccbin", CXX, "-Xcompiler", "-fPIC,-ffp-contract=off",
-               "--expt-relaxed-constexpr", "--split-compile=4"] + ARCH
+               "--expt-relaxed-constexpr"] + ARCH
 CU_SOURCES = {
     "solve.cu": [],
     "cycle_single.cu": [],

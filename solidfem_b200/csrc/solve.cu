@@ -547,6 +547,10 @@ sf_status solver_enqueue_iteration(DeviceSolver& s) {
     launch_body<pcg_update_kernel>(grid_for_reduction(s.n), kReduceThreads, 0, st, s.n, s.p, s.ap, s.x, s.r, s.partials, s.state);
     launch_body<sell_pcg_check_kernel>(grid, kThreads, 0, st, A, s.x, s.rhs, s.r, s.partials, s.state);
   } else switch (s.system.lanes_per_row) {
+    // Short rows (under about 7 blocks, raw sparse systems) take teams of eight as well: a row of up
+    // to eight blocks is summed in the order of 32 lanes, whose other lanes add zeros, with four rows
+    // to a warp instead of one (45^3 cells under Jacobi: 39 -> 33 us an iteration).
+    case 4:
     case 8: launch_pcg_spmv_lpr<8>(s); break;
     case 16: launch_pcg_spmv_lpr<16>(s); break;
     default: launch_pcg_spmv_lpr<32>(s); break;
