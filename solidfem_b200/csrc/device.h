@@ -82,8 +82,10 @@ bool wants_sell(const DevBsr& m, uint64_t sell_min_rows);
 bool wants_split(const DevBsr& m, bool uniform_lanes);
 
 // Splits the rows of a block matrix into groups of at most `target` value bytes (a longer row is
-// a group of its own) and chooses the lanes per row from the mean blocks per row.
-sf_status make_row_groups(struct DeviceSolver& s, DevBsr& m, const uint32_t* host_starts, size_t value_bytes);
+// a group of its own) and chooses the lanes per row from the mean blocks per row. `one_pass`: no
+// more rows to a group than a warp multiplies at once.
+sf_status make_row_groups(struct DeviceSolver& s, DevBsr& m, const uint32_t* host_starts, size_t value_bytes,
+                          bool one_pass = false);
 
 // The solver's scalar state, resident on the device so the iteration loop runs without host
 // round trips; kernels read `status` and exit early once the solve has ended.
@@ -170,6 +172,8 @@ struct LaunchRecord {
   dim3 grid, block;
   size_t smem = 0;
   unsigned cluster = 0;  // CTAs per thread-block cluster (grid.x), 0 for a plain launch
+  unsigned capacity = 0;  // a row-group walk (any grid gives the same bits): the blocks the device holds at once
+  bool fixed_blocks = false;  // the pack opens with the block count its sums are formed for
   std::vector<unsigned char> pack;
 };
 extern thread_local std::vector<LaunchRecord>* g_recorder;

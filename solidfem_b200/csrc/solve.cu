@@ -28,9 +28,17 @@ template <int LPR>
 void launch_pcg_spmv_lpr(DeviceSolver& s) {
   Op<double> A = op_of<double>(s.system);
   Shape sh = shape_of(A, true);
-  launch_body<pcg_spmv_dot_kernel<LPR>>(sh.grid, sh.threads, sh.smem, s.stream, A, s.p, s.ap, s.partials, s.state);
+  // (outside a batch the grid is the block count)
+  auto fixed = [&](LaunchRecord& r) {
+    r.capacity = (unsigned)sh.capacity;
+    r.fixed_blocks = true;
+  };
+  launch_body<pcg_spmv_dot_kernel<LPR>>(sh.grid, sh.threads, sh.smem, s.stream, (uint32_t)sh.grid, A, s.p, s.ap, s.partials, s.state);
+  if (g_recorder) fixed(g_recorder->back());
   launch_body<pcg_update_kernel>(grid_for_reduction(s.n), kReduceThreads, 0, s.stream, s.n, s.p, s.ap, s.x, s.r, s.partials, s.state);
-  launch_body<pcg_check_kernel<LPR>>(sh.grid, sh.threads, sh.smem, s.stream, A, s.x, s.rhs, s.r, s.partials, s.state);
+  launch_body<pcg_check_kernel<LPR>>(sh.grid, sh.threads, sh.smem, s.stream, (uint32_t)sh.grid, A, s.x, s.rhs, s.r,
+                                     s.partials, s.state);
+  if (g_recorder) fixed(g_recorder->back());
 }
 
 }  // namespace
@@ -187,7 +195,7 @@ void dev_free_all(DeviceSolver& s) {
   s.bytes = 0;
 }
 
-sf_status make_row_groups(DeviceSolver& s, DevBsr& m, const uint32_t* starts, size_t value_bytes) {
+sf_status make_row_groups(DeviceSolver& s, DevBsr& m, const uint32_t* starts, size_t value_bytes, bool one_pass) {
   // Rows per group: as many mean rows as fit kGroupTarget bytes (1 to 8, a power of two). The
   // warp splits into that many teams of 32 / teams lanes, one row each, so a warp works on several
   // light rows at once (their x gathers and epilogue loads overlap) and on a heavy row whole.
@@ -208,7 +216,7 @@ sf_status make_row_groups(DeviceSolver& s, DevBsr& m, const uint32_t* starts, si
   while (r < m.rows) {
     uint32_t e = r + 1;
     size_t bytes = (size_t)(starts[e] - starts[r]) * value_bytes;
-    while (e < m.rows && bytes + (size_t)(starts[e + 1] - starts[e]) * value_bytes <= target) {
+    while (e < m.rows && (!one_pass || e - r < (uint32_t)teams) && bytes + (size_t)(starts[e + 1] - starts[e]) * value_bytes <= target) {
       bytes += (size_t)(starts[e + 1] - starts[e]) * value_bytes;
       ++e;
     }
@@ -371,7 +379,10 @@ sf_status device_bsr(DeviceSolver& s, const Bsr& h, DevBsr& d, bool alias) {
     if (sf_status e = dev_alloc(s, &d.vals, std::max<size_t>(1, n) * sizeof(S))) return e;
     if (sf_status e = setup_convert<S>(s.stream, n, h.dev, (S*)d.vals)) return e;
   }
-  if (sf_status e = make_row_groups(s, d, h.starts.data(), h.rb * h.cb * sizeof(S))) return e;
+  // A level's products keep a group to the rows a warp takes in one pass: five or six short rows to
+  // a group of four teams cost two passes, the second mostly idle. (The f64 system's groups also
+  // order its dot products' sums, so they stay as they are.)
+  if (sf_status e = make_row_groups(s, d, h.starts.data(), h.rb * h.cb * sizeof(S), true)) return e;
   if (wants_split(d, s.uniform_lanes)) {
     if (sf_status e = make_split_converted<S>(s, d, h.starts.data(), h.dev)) return e;
   } else if (wants_sell(d, s.sell_min_rows)) {
@@ -644,8 +655,11 @@ sf_status batch_build(const std::vector<DeviceSolver*>& inst, cudaStream_t strea
     // Block sizes may differ (a row-group kernel's warps per block follow its largest group); the
     // bodies work with any block size and place each warp's staging slot by their own operator,
     // so the batch takes the largest block and the largest per-warp slot.
-    size_t per_warp = 0;
+    size_t per_warp = 0, blocks = 0;
+    unsigned capacity = ~0u;
     for (size_t i = 0; i < inst.size(); ++i) {
+      blocks += rec[i][j].grid.x;
+      capacity = std::min(capacity, rec[i][j].capacity);
       t.grid.x = std::max(t.grid.x, rec[i][j].grid.x);
       t.block.x = std::max(t.block.x, rec[i][j].block.x);
       per_warp = std::max(per_warp, rec[i][j].smem / std::max(1u, rec[i][j].block.x / 32));
@@ -660,6 +674,18 @@ sf_status batch_build(const std::vector<DeviceSolver*>& inst, cudaStream_t strea
       t.block.x = (unsigned)(32 * warps);
     }
     if (!t.cluster) t.smem = per_warp * (t.block.x / 32);
+    // A row-group walk of more blocks than the device holds takes what it holds, shared among the
+    // instances: a warp then walks several groups, each staged while the one before is multiplied,
+    // instead of one group a warp whose staging nothing hides (16 cantilevers of 9,720 to 11,178
+    // unknowns: 305 -> 270 us an iteration, the groups' single pass included).
+    // The bodies with sums run the blocks these are formed for (the largest instance's, as before) in
+    // turn, so their bits stay.
+    if (rec[0][j].fixed_blocks) {
+      const uint32_t count = t.grid.x;
+      for (size_t i = 0; i < inst.size(); ++i) std::memcpy(host.data() + i * bytes, &count, sizeof(count));
+    }
+    if (capacity && blocks > capacity)
+      t.grid.x = std::min<unsigned>(t.grid.x, (capacity + (unsigned)inst.size() - 1) / (unsigned)inst.size());
     if (t.smem > 200 * 1024) {
       batch_destroy(out);
       return fail(SF_INVALID_ARGUMENT, "a study of the batch needs more shared memory per warp than one SM holds");
@@ -982,7 +1008,7 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(Op<double> A, const do
   epi.p = x + off;
   epi.ap = y + off;
   epi.local = 0.0;
-  run_groups<double, double, 3, 3, LPR, false>(A, x + off, wbase, epi, OpenGate{});
+  run_groups<double, double, 3, 3, LPR, false>(A, x + off, wbase, epi, OpenGate{}, blockIdx.x, gridDim.x);
   energy_finish(epi.local, scratch, energy);
 }
 

@@ -345,15 +345,16 @@ struct CheckGate {
 // With MAG it also sums |a_ij x_j| per row (the rounding floor of pcg.rs:246-248). A group is
 // staged one grid-stride step ahead (double buffer), its descriptor two steps ahead.
 // Returns the gate (uniform over the grid: a body may still reduce across its blocks after true).
+// The walk is that of block `block` of `blocks`: a body's own, or one of several it runs in turn.
 template <typename S, typename V, int RB, int CB, int LPR, bool MAG, class Epi, class Gate>
 __device__ __forceinline__ bool run_groups(const Op<S>& A, const V* __restrict__ x, char* wbase, Epi& epi,
-                                           const Gate& gate) {
+                                           const Gate& gate, uint32_t block, uint32_t blocks) {
   constexpr int LEN = RB * CB;
   constexpr int TEAMS = 32 / LPR;
   const int lane = threadIdx.x & 31;
   const int team = lane / LPR, tl = lane % LPR;
-  const uint32_t nw = gridDim.x * (blockDim.x >> 5);
-  uint32_t g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t nw = blocks * (blockDim.x >> 5);
+  uint32_t g = block * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const uint32_t sb = slot_bytes(A);
   int vo0 = 0, vo1 = 0, co0 = 0, co1 = 0, so0 = 0, so1 = 0;
   auto issue = [&](const uint4& d, int slot) {
@@ -525,7 +526,7 @@ __device__ __forceinline__ void bsr_kernel(Op<S> A, const V* __restrict__ x, V* 
   extern __shared__ __align__(16) char smem[];
   char* wbase = smem + (threadIdx.x >> 5) * 2 * slot_bytes(A);
   EpiAxpy<V, RB, LPR, OP> epi{y, b, {}};
-  run_groups<S, V, RB, CB, LPR, false>(A, x, wbase, epi, StatusGate{status});
+  run_groups<S, V, RB, CB, LPR, false>(A, x, wbase, epi, StatusGate{status}, blockIdx.x, gridDim.x);
 }
 
 // One Chebyshev step fused with its product (cycle.rs:611-650): ad = A d_old; r -= ad;
@@ -602,7 +603,7 @@ __device__ __forceinline__ void cheb_step_kernel(Op<S> A, const S* __restrict__ 
   epi.outer = outer;
   epi.keep = keep;
   epi.step = step;
-  run_groups<S, V, RB, RB, LPR, false>(A, d_old, wbase, epi, StatusGate{status});
+  run_groups<S, V, RB, RB, LPR, false>(A, d_old, wbase, epi, StatusGate{status}, blockIdx.x, gridDim.x);
 }
 
 // The smoother's start from a zero guess (cycle.rs:591-610): r = b; d = (D^-1 b) / theta; x = d.
@@ -707,14 +708,20 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 
 // Each block writes its partials; the last block to finish sums them in block order.
 template <int K>
-__device__ __forceinline__ bool finish_partials(double (&v)[K], double* partials, unsigned* ticket, double (&total)[K]) {
+__device__ __forceinline__ void store_partials(double (&v)[K], double* partials, uint32_t block, uint32_t blocks) {
   __shared__ double sh[32];
-  __shared__ bool last;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     double s = block_sum(v[k], sh);
-    if (threadIdx.x == 0) partials[(size_t)k * gridDim.x + blockIdx.x] = s;
+    if (threadIdx.x == 0) partials[(size_t)k * blocks + block] = s;
   }
+}
+
+// True in the last block of the grid to arrive, with the sums of `blocks` partials in its warp 0.
+template <int K>
+__device__ __forceinline__ bool sum_partials(double* partials, uint32_t blocks, unsigned* ticket, double (&total)[K]) {
+  __shared__ double sh[32];
+  __shared__ bool last;
   if (threadIdx.x == 0) {
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x - 1;
@@ -725,11 +732,17 @@ __device__ __forceinline__ bool finish_partials(double (&v)[K], double* partials
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     double s = 0.0;
-    for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) s += __ldcg(partials + (size_t)k * gridDim.x + i);
+    for (unsigned i = threadIdx.x; i < blocks; i += blockDim.x) s += __ldcg(partials + (size_t)k * blocks + i);
     total[k] = block_sum(s, sh);
   }
   if (threadIdx.x == 0) *ticket = 0u;
   return true;
+}
+
+template <int K>
+__device__ __forceinline__ bool finish_partials(double (&v)[K], double* partials, unsigned* ticket, double (&total)[K]) {
+  store_partials<K>(v, partials, blockIdx.x, gridDim.x);
+  return sum_partials<K>(partials, gridDim.x, ticket, total);
 }
 
 // ------------------------------------------------------------ SELL-32: one thread per row
@@ -1784,7 +1797,7 @@ __device__ __forceinline__ void bsr_start_kernel(Op<S> A, const V* __restrict__ 
   EpiStart<S, V, RB, LPR, OP> epi;
   epi.a = a;
   epi.b = b;
-  run_groups<S, V, RB, CB, LPR, false>(A, x, wbase, epi, StatusGate{status});
+  run_groups<S, V, RB, CB, LPR, false>(A, x, wbase, epi, StatusGate{status}, blockIdx.x, gridDim.x);
 }
 
 struct SellDot {
@@ -1904,19 +1917,24 @@ struct EpiDot {
 };
 
 // ap = A p on the f64 system with the curvature p.ap; then alpha = rz / curvature
-// (pcg.rs:217-228).
+// (pcg.rs:217-228). `blocks` fixes the partials and with them the sum's bits; a grid of fewer
+// blocks (a batch's, where many studies share the device) runs several of them each in turn.
 template <int LPR>
-__device__ __forceinline__ void pcg_spmv_dot_kernel(Op<double> A, const double* __restrict__ p,
+__device__ __forceinline__ void pcg_spmv_dot_kernel(uint32_t blocks, Op<double> A, const double* __restrict__ p,
                                                                  double* __restrict__ ap, double* partials, PcgState* st) {
   extern __shared__ __align__(16) char smem[];
   char* wbase = smem + (threadIdx.x >> 5) * 2 * slot_bytes(A);
   EpiDot<LPR> epi;
   epi.p = p;
   epi.ap = ap;
-  epi.local = 0.0;
-  if (!run_groups<double, double, 3, 3, LPR, false>(A, p, wbase, epi, StatusGate{&st->status})) return;
-  double v[1] = {epi.local}, total[1];
-  if (finish_partials<1>(v, partials, &st->tickets[0], total) && threadIdx.x == 0) {
+  for (uint32_t b = blockIdx.x; b < blocks; b += gridDim.x) {
+    epi.local = 0.0;
+    if (!run_groups<double, double, 3, 3, LPR, false>(A, p, wbase, epi, StatusGate{&st->status}, b, blocks)) return;
+    double v[1] = {epi.local};
+    store_partials<1>(v, partials, b, blocks);
+  }
+  double total[1];
+  if (sum_partials<1>(partials, blocks, &st->tickets[0], total) && threadIdx.x == 0) {
     double curvature = total[0];
     st->curvature = curvature;
     if (isnan(curvature) || curvature <= 0.0 || !isfinite(st->rz)) {
@@ -2004,7 +2022,7 @@ struct EpiCheck {
 // The true residual when the recursive one reports convergence, with the rounding floor of the
 // product (pcg.rs:234-255): r = b - A x; converge, or restart from it.
 template <int LPR>
-__device__ __forceinline__ void pcg_check_kernel(Op<double> A, const double* __restrict__ x,
+__device__ __forceinline__ void pcg_check_kernel(uint32_t blocks, Op<double> A, const double* __restrict__ x,
                                                               const double* __restrict__ b, double* __restrict__ r,
                                                               double* partials, PcgState* st) {
   extern __shared__ __align__(16) char smem[];
@@ -2013,11 +2031,15 @@ __device__ __forceinline__ void pcg_check_kernel(Op<double> A, const double* __r
   epi.b = b;
   epi.r = r;
   epi.starts = A.starts;
-  epi.res2 = 0.0;
-  epi.bound2 = 0.0;
-  if (!run_groups<double, double, 3, 3, LPR, true>(A, x, wbase, epi, CheckGate{st})) return;
-  double v[2] = {epi.res2, epi.bound2}, total[2];
-  if (finish_partials<2>(v, partials, &st->tickets[2], total) && threadIdx.x == 0) {
+  for (uint32_t k = blockIdx.x; k < blocks; k += gridDim.x) {
+    epi.res2 = 0.0;
+    epi.bound2 = 0.0;
+    if (!run_groups<double, double, 3, 3, LPR, true>(A, x, wbase, epi, CheckGate{st}, k, blocks)) return;
+    double v[2] = {epi.res2, epi.bound2};
+    store_partials<2>(v, partials, k, blocks);
+  }
+  double total[2];
+  if (sum_partials<2>(partials, blocks, &st->tickets[2], total) && threadIdx.x == 0) {
     double rel = sqrt(total[0]) / st->rhs_norm;
     double floor = sqrt(total[1]) / st->rhs_norm;
     st->rel = rel;
@@ -2228,6 +2250,7 @@ int grid_for_reduction(size_t n) {
 struct Shape {
   int threads, grid;
   size_t smem;
+  int capacity;  // blocks the device holds at once
 };
 
 template <typename S>
@@ -2240,15 +2263,22 @@ Shape shape_of(const Op<S>& A, bool reduction) {
   size_t want = (A.ngroups + warps - 1) / warps;
   size_t grid = std::min<size_t>(want, (size_t)sm_count() * per_sm);
   if (reduction) grid = std::min<size_t>(grid, (size_t)kReduceBlocks * 2);
-  return {32 * warps, (int)std::max<size_t>(1, grid), smem};
+  return {32 * warps, (int)std::max<size_t>(1, grid), smem, sm_count() * per_sm};
 }
 
+
+// A row-group walk without a reduction: its bits do not depend on the grid.
+template <auto Body, typename... A>
+void launch_groups(const Shape& sh, cudaStream_t st, A&&... args) {
+  launch_body<Body>(sh.grid, sh.threads, sh.smem, st, std::forward<A>(args)...);
+  if (g_recorder) g_recorder->back().capacity = (unsigned)sh.capacity;
+}
 
 template <typename S, typename V, int RB, int CB, int LPR, int OP>
 void launch_bsr_lpr(const DevBsr& m, const V* x, V* y, const V* b, const int* status, cudaStream_t st) {
   Op<S> A = op_of<S>(m);
   Shape sh = shape_of(A, false);
-  launch_body<bsr_kernel<S, V, RB, CB, LPR, OP>>(sh.grid, sh.threads, sh.smem, st, A, x, y, b, status);
+  launch_groups<bsr_kernel<S, V, RB, CB, LPR, OP>>(sh, st, A, x, y, b, status);
 }
 
 // The SELL-32 and split-row products run in blocks of two warps. The resident warps per SM do not
@@ -2324,7 +2354,7 @@ void launch_cheb_step_lpr(const DevLevel& L, const V* d_old, V* d_new, V* r, V* 
                           const int* status, cudaStream_t st) {
   Op<S> A = op_of<S>(L.a);
   Shape sh = shape_of(A, false);
-  launch_body<cheb_step_kernel<S, V, RB, LPR>>(sh.grid, sh.threads, sh.smem, st, A, (const S*)L.dinv, d_old, d_new, r,
+  launch_groups<cheb_step_kernel<S, V, RB, LPR>>(sh, st, A, (const S*)L.dinv, d_old, d_new, r,
                                                 x, outer, (V)keep, (V)step, status);
 }
 
@@ -2377,10 +2407,10 @@ void launch_start_rb(const DevBsr& m, const V* x, const V* b, const StartArgs<S,
   Op<S> A = op_of<S>(m);
   Shape sh = shape_of(A, false);
   switch (m.lanes_per_row) {
-    case 4: launch_body<bsr_start_kernel<S, V, RB, CB, 4, OP>>(sh.grid, sh.threads, sh.smem, st, A, x, b, a, status); break;
-    case 8: launch_body<bsr_start_kernel<S, V, RB, CB, 8, OP>>(sh.grid, sh.threads, sh.smem, st, A, x, b, a, status); break;
-    case 16: launch_body<bsr_start_kernel<S, V, RB, CB, 16, OP>>(sh.grid, sh.threads, sh.smem, st, A, x, b, a, status); break;
-    default: launch_body<bsr_start_kernel<S, V, RB, CB, 32, OP>>(sh.grid, sh.threads, sh.smem, st, A, x, b, a, status); break;
+    case 4: launch_groups<bsr_start_kernel<S, V, RB, CB, 4, OP>>(sh, st, A, x, b, a, status); break;
+    case 8: launch_groups<bsr_start_kernel<S, V, RB, CB, 8, OP>>(sh, st, A, x, b, a, status); break;
+    case 16: launch_groups<bsr_start_kernel<S, V, RB, CB, 16, OP>>(sh, st, A, x, b, a, status); break;
+    default: launch_groups<bsr_start_kernel<S, V, RB, CB, 32, OP>>(sh, st, A, x, b, a, status); break;
   }
 }
 
