@@ -239,6 +239,11 @@ sf_status build_box_mesh(const double origin[3], const double size[3], const uin
 // QuadraticTetMesh::face_connected_bodies, quadratic.rs:129-166.
 vector<vector<uint32_t>> face_connected_bodies(const Mesh& mesh) {
   size_t n = mesh.tets.size();
+  if (mesh.one_body && n) {
+    vector<vector<uint32_t>> all(1, vector<uint32_t>(n));
+    std::iota(all[0].begin(), all[0].end(), 0u);
+    return all;
+  }
   vector<size_t> parent(n);
   std::iota(parent.begin(), parent.end(), 0);
   auto find = [&](size_t x) {

@@ -454,6 +454,46 @@ __global__ void face_bucket_kernel(const uint32_t* __restrict__ off, unsigned lo
   }
 }
 
+// Joins the two tetrahedra of every shared face (equal neighbours in a sorted bucket): a union-find
+// whose roots are only ever hooked under smaller ones, so each body ends under its smallest tet.
+__device__ __forceinline__ uint32_t body_root(uint32_t* parent, uint32_t t) {
+  volatile uint32_t* p = parent;
+  for (uint32_t up = p[t]; up != t; up = p[t]) {
+    const uint32_t over = p[up];
+    if (over != up) p[t] = over;  // halve the path; over is an ancestor, whoever else writes
+    t = up;
+  }
+  return t;
+}
+__global__ void body_start_kernel(uint32_t* __restrict__ parent, size_t ntets) {
+  GRID_STRIDE(t, ntets) parent[t] = (uint32_t)t;
+}
+__global__ void body_join_kernel(const uint32_t* __restrict__ off, const unsigned long long* __restrict__ rest,
+                                 const uint32_t* __restrict__ item, uint32_t* parent, size_t n) {
+  GRID_STRIDE(a, n) {
+    for (uint32_t i = off[a]; i + 1 < off[a + 1]; ++i) {
+      if (rest[i] != rest[i + 1]) continue;
+      uint32_t x = item[i] / 4, y = item[i + 1] / 4;
+      for (;;) {
+        x = body_root(parent, x);
+        y = body_root(parent, y);
+        if (x == y) break;
+        if (x < y) {
+          const uint32_t t = x;
+          x = y;
+          y = t;
+        }
+        if (atomicCAS(parent + x, x, y) == x) break;  // x was still a root: it now hangs under y < x
+      }
+    }
+  }
+}
+__global__ void body_count_kernel(const uint32_t* __restrict__ parent, size_t ntets, uint32_t* roots) {
+  uint32_t mine = 0;
+  GRID_STRIDE(t, ntets) mine += parent[t] == (uint32_t)t;
+  if (mine) atomicAdd(roots, mine);
+}
+
 __global__ void face_emit_kernel(const uint32_t* __restrict__ off, const unsigned long long* __restrict__ rest,
                                  const uint32_t* __restrict__ item, const uint32_t* __restrict__ soff,
                                  const uint32_t* __restrict__ tets10, sf_boundary_face* __restrict__ faces, size_t n) {
@@ -646,7 +686,17 @@ sf_status from_linear(Build& b, double* pos, size_t n, uint32_t* corners, size_t
   if (cudaError_t e = cudaStreamSynchronize(st)) return cuda_fail(e, "mesh faces");
   if (manifold) return fail(SF_MESH_NON_MANIFOLD_FACE, "a face is shared by more than two tetrahedra");
   sf_boundary_face* faces = b.alloc<sf_boundary_face>(nfaces);
+  uint32_t* parent = b.alloc<uint32_t>(ntets);
+  uint32_t* roots = b.alloc<uint32_t>(1);
   if (b.err) return cuda_fail(b.err, "mesh build");
+  // whether the mesh is one face-connected body (the usual case), which spares every study of it
+  // the host's search for bodies (10 ms of the gate plate's creation)
+  cudaMemsetAsync(roots, 0, 4, st);
+  body_start_kernel<<<grid_of(ntets), kT, 0, st>>>(parent, ntets);
+  body_join_kernel<<<grid_of(n), kT, 0, st>>>(foff, rest, item, parent, n);
+  body_count_kernel<<<grid_of(ntets), kT, 0, st>>>(parent, ntets, roots);
+  uint32_t bodies = 0;
+  cudaMemcpyAsync(&bodies, roots, 4, cudaMemcpyDeviceToHost, st);
   face_emit_kernel<<<grid_of(n), kT, 0, st>>>(foff, rest, item, soff, mirror->tets, faces, n);
   // host arrays
   out = Mesh();
@@ -663,6 +713,7 @@ sf_status from_linear(Build& b, double* pos, size_t n, uint32_t* corners, size_t
   if (cudaError_t e = cudaGetLastError()) return cuda_fail(e, "mesh kernels");
   mirror->stream = nullptr;
   out.dev = mirror;
+  out.one_body = bodies == 1;
   drain.armed = false;  // the copies above synchronized the stream
   return SF_OK;
 }

@@ -50,6 +50,7 @@ struct Mesh {
   size_t vertex_count = 0;
   vector<sf_boundary_face> faces;  // sorted by their sorted corners
   std::shared_ptr<DeviceMesh> dev;  // set when the mesh was built on a device
+  bool one_body = false;            // known to be one face-connected body (found by a device build)
 };
 
 sf_status build_box_mesh(const double origin[3], const double size[3], const uint64_t div[3],
@@ -139,6 +140,10 @@ struct HostLevel {
   Bsr p;
   bool has_factor = false;
   size_t factor_n = 0;
+  // P's transpose on the device, as the Galerkin product made it, until the solver takes it over:
+  // row starts (and on the host), fine rows, and the P block each one is.
+  vector<uint32_t> t_starts;
+  uint32_t *dev_t_starts = nullptr, *dev_t_rows = nullptr, *dev_t_at = nullptr;
   double* dev_coarse_inverse = nullptr;  // the dense inverse of the coarsest level, row-major f64, device
   vector<uint32_t> aggregates;
 };
