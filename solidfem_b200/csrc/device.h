@@ -224,6 +224,14 @@ size_t setup_norm_scratch(size_t n);
 sf_status setup_start_vector(cudaStream_t st, size_t n, double* v);
 sf_status setup_normalize(cudaStream_t st, size_t n, const double* src, void* scratch, double* norm, double* v);
 sf_status setup_entry_rows(cudaStream_t st, uint32_t rows, const uint32_t* starts, uint32_t* out);
+// The transpose of a pattern of `entries` block columns below `width`: the columns' counts (zeros
+// before), then, with the starts they give and a copy of them as cursors, each column's entries in
+// ascending order and their rows. No column may have more than kTransposeLongest entries.
+static const uint32_t kTransposeLongest = 8192;
+sf_status setup_column_counts(cudaStream_t st, size_t entries, const uint32_t* cols, uint32_t* counts);
+sf_status setup_transpose_pattern(cudaStream_t st, size_t entries, const uint32_t* cols, const uint32_t* entry_row,
+                                  uint32_t width, uint32_t longest, const uint32_t* t_starts, uint32_t* cursors,
+                                  uint32_t* t_at, uint32_t* t_rows);
 // The geometric strength graph (aggregate.rs:53-69): with out_starts null, each row's strong count
 // into out and its closest squared distance into closest; else the strong columns at out_starts.
 sf_status setup_strength(cudaStream_t st, uint32_t rows, const uint32_t* starts, const uint32_t* cols, const double* pos,

@@ -177,9 +177,11 @@ struct SetupMachine {
 
   // A union pattern (the symbolic_rows of a product) on the device: a count pass, the row starts
   // by a prefix sum here, a fill pass. `out` gets the device starts and columns and the same
-  // arrays on the host, equal to what symbolic_rows gives (each row's distinct columns, sorted).
+  // arrays on the host (the columns where they are read there), equal to what symbolic_rows gives
+  // (each row's distinct columns, sorted).
   sf_status device_union(size_t rows, size_t width, const uint32_t* d_outer_starts, const uint32_t* d_outer_idx,
-                         bool self, const uint32_t* d_inner_starts, const uint32_t* d_inner_cols, Bsr& out) {
+                         bool self, const uint32_t* d_inner_starts, const uint32_t* d_inner_cols, Bsr& out,
+                         bool host_columns = true) {
     sf_status e = dev_alloc(dev, (void**)&out.dev_starts, (rows + 1) * 4);
     if (!e)
       e = setup_union_rows(dev.stream, (uint32_t)rows, (uint32_t)width, d_outer_starts, d_outer_idx, self,
@@ -194,10 +196,10 @@ struct SetupMachine {
     if ((e = dev_alloc(dev, (void**)&out.dev_cols, std::max<size_t>(1, total) * 4))) return e;
     e = setup_union_rows(dev.stream, (uint32_t)rows, (uint32_t)width, d_outer_starts, d_outer_idx, self,
                          d_inner_starts, d_inner_cols, out.dev_starts, out.dev_cols);
+    if (!host_columns || e) return e;
     out.cols.resize(total);
-    if (!e && total) copy_d2h(dev, out.cols.data(), out.dev_cols, total * 4);
-    if (!e) e = sync("union pattern");
-    return e;
+    if (total) copy_d2h(dev, out.cols.data(), out.dev_cols, total * 4);
+    return sync("union pattern");
   }
 
   // setup.rs:269-321 on the device; the block norms for the join pass come back to the host.
@@ -524,7 +526,7 @@ struct SetupMachine {
 
   // The row of every entry of a pattern, on the device.
   sf_status entry_rows(const Bsr& m, uint32_t** out) {
-    if (sf_status e = dev_alloc(dev, (void**)out, std::max<size_t>(1, m.cols.size()) * 4)) return e;
+    if (sf_status e = dev_alloc(dev, (void**)out, std::max<size_t>(1, m.starts.back()) * 4)) return e;
     return setup_entry_rows(dev.stream, (uint32_t)m.rows, m.dev_starts, *out);
   }
 
@@ -581,7 +583,7 @@ struct SetupMachine {
     sf_status e = SF_OK;
     if (union_on_device(aggregates)) {
       e = device_union(rows, aggregates, current.dev_starts, current.dev_cols, false, prolongator.dev_starts,
-                       prolongator.dev_cols, ap);
+                       prolongator.dev_cols, ap, false);
     } else {
       symbolic_rows(
           rows, aggregates, opt.threads,
@@ -596,7 +598,7 @@ struct SetupMachine {
       e = upload_pattern(ap);
     }
     uint32_t* rows_of = nullptr;
-    size_t entries = ap.cols.size();
+    size_t entries = ap.starts.back();
     if (!e) e = dev_alloc(dev, (void**)&ap.dev, std::max<size_t>(1, entries) * rb * MODES * 8);
     if (!e) e = entry_rows(ap, &rows_of);
     if (!e)
@@ -609,27 +611,63 @@ struct SetupMachine {
     return SF_OK;
   }
 
+  // P's pattern by columns, fine rows ascending, and where each block lies in P: on the device, the
+  // row starts also on the host (and the fine rows, where the coarse pattern is made there). A
+  // column too long for the device's sort takes the whole pattern to the host's counting sort.
+  sf_status transpose_prolongator(vector<uint32_t>& starts, vector<uint32_t>& rows, uint32_t** d_starts,
+                                  uint32_t** d_rows, uint32_t** d_at) {
+    const size_t entries = prolongator.starts.back();
+    uint32_t *cursors = nullptr, *rows_of = nullptr;
+    starts.assign(aggregates + 1, 0);
+    sf_status e = dev_alloc(dev, (void**)d_starts, (aggregates + 1) * 4);  // zeros
+    if (!e) e = setup_column_counts(dev.stream, entries, prolongator.dev_cols, *d_starts);
+    if (!e) copy_d2h(dev, starts.data() + 1, *d_starts, aggregates * 4);
+    if (!e) e = sync("transpose counts");
+    if (e) return e;
+    uint32_t longest = 0;
+    for (size_t i = 0; i < aggregates; ++i) {
+      longest = std::max(longest, starts[i + 1]);
+      starts[i + 1] += starts[i];
+    }
+    const bool host = longest > kTransposeLongest || !union_on_device(aggregates);
+    if (!e) e = dev_alloc(dev, (void**)d_rows, std::max<size_t>(1, entries) * 4);
+    if (!e) e = dev_alloc(dev, (void**)d_at, std::max<size_t>(1, entries) * 4);
+    if (e) return e;
+    copy_h2d(dev, *d_starts, starts.data(), (aggregates + 1) * 4);
+    if (host) {
+      vector<uint32_t> filled(starts.begin(), starts.end() - 1), at(entries);
+      rows.resize(entries);
+      for (size_t row = 0; row < prolongator.rows; ++row)
+        for (uint32_t k = prolongator.starts[row]; k < prolongator.starts[row + 1]; ++k) {
+          const uint32_t o = filled[prolongator.cols[k]]++;
+          rows[o] = (uint32_t)row;
+          at[o] = k;
+        }
+      copy_h2d(dev, *d_rows, rows.data(), entries * 4);
+      copy_h2d(dev, *d_at, at.data(), entries * 4);
+      return sync("transpose");
+    }
+    e = dev_alloc(dev, (void**)&cursors, std::max<size_t>(1, aggregates) * 4);
+    if (!e) e = entry_rows(prolongator, &rows_of);
+    if (!e) {
+      cudaMemcpyAsync(cursors, *d_starts, aggregates * 4, cudaMemcpyDeviceToDevice, dev.stream);
+      e = setup_transpose_pattern(dev.stream, entries, prolongator.dev_cols, rows_of, (uint32_t)aggregates, longest,
+                                  *d_starts, cursors, *d_at, *d_rows);
+    }
+    dev_free(dev, cursors);
+    dev_free(dev, rows_of);
+    return e;
+  }
+
   // P^T (A P) by coarse row, P read by columns with fine rows ascending (transfer.rs:173-238).
   sf_status run_galerkin() {
     const size_t cdim = MODES;
-    vector<uint32_t> pt_starts(aggregates + 1, 0);
-    for (uint32_t c : prolongator.cols) pt_starts[c + 1] += 1;
-    for (size_t i = 0; i < aggregates; ++i) pt_starts[i + 1] += pt_starts[i];
-    vector<uint32_t> filled(pt_starts.begin(), pt_starts.end() - 1);
-    vector<uint32_t> pt_rows(prolongator.cols.size()), pt_at(prolongator.cols.size());
-    for (size_t row = 0; row < prolongator.rows; ++row)
-      for (uint32_t at = prolongator.starts[row]; at < prolongator.starts[row + 1]; ++at) {
-        uint32_t o = filled[prolongator.cols[at]]++;
-        pt_rows[o] = (uint32_t)row;
-        pt_at[o] = at;
-      }
     coarse = Bsr();
     coarse.rows = aggregates;
     coarse.rb = coarse.cb = cdim;
+    vector<uint32_t> pt_starts, pt_rows;
     uint32_t *d_pt_starts = nullptr, *d_pt_rows = nullptr, *d_pt_at = nullptr, *rows_of = nullptr;
-    sf_status e = upload(pt_starts, &d_pt_starts);
-    if (!e) e = upload(pt_rows, &d_pt_rows);
-    if (!e) e = upload(pt_at, &d_pt_at);
+    sf_status e = transpose_prolongator(pt_starts, pt_rows, &d_pt_starts, &d_pt_rows, &d_pt_at);
     if (!e && union_on_device(aggregates)) {
       e = device_union(aggregates, aggregates, d_pt_starts, d_pt_rows, false, ap.dev_starts, ap.dev_cols, coarse);
     } else if (!e) {
@@ -651,10 +689,17 @@ struct SetupMachine {
       e = setup_galerkin(dev.stream, (int)prolongator.rb, entries, rows_of, coarse.dev_cols, d_pt_starts, d_pt_rows,
                          d_pt_at, prolongator.dev, ap.dev_starts, ap.dev_cols, ap.dev, coarse.dev);
     if (!e) e = sync("galerkin");
-    for (void* p : {(void*)d_pt_starts, (void*)d_pt_rows, (void*)d_pt_at, (void*)rows_of}) dev_free(dev, p);
+    dev_free(dev, rows_of);
     release(ap);
-    if (e) return e;
+    if (e) {
+      for (void* p : {(void*)d_pt_starts, (void*)d_pt_rows, (void*)d_pt_at}) dev_free(dev, p);
+      return e;
+    }
     HostLevel lv;
+    lv.t_starts = std::move(pt_starts);  // the solver restricts with this transpose
+    lv.dev_t_starts = d_pt_starts;
+    lv.dev_t_rows = d_pt_rows;
+    lv.dev_t_at = d_pt_at;
     lv.a = std::move(current);
     lv.inverse_diagonal = inv;
     inv = nullptr;

@@ -438,6 +438,37 @@ __global__ void entry_rows_kernel(uint32_t rows, const uint32_t* __restrict__ st
     for (uint32_t j = starts[row]; j < starts[row + 1]; ++j) out[j] = row;
 }
 
+// The transpose's parts: column counts; each entry into its column's list in any order; then a block
+// per column puts its list in ascending order (an entry's place is the number of smaller ones, read
+// from shared memory: lists hold tens to hundreds of entries) and adds the entries' rows.
+__global__ void column_counts_kernel(size_t entries, const uint32_t* __restrict__ cols, uint32_t* counts) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < entries; i += (size_t)gridDim.x * blockDim.x)
+    atomicAdd(counts + cols[i], 1u);
+}
+__global__ void transpose_fill_kernel(size_t entries, const uint32_t* __restrict__ cols, uint32_t* cursors,
+                                      uint32_t* __restrict__ at) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < entries; i += (size_t)gridDim.x * blockDim.x)
+    at[atomicAdd(cursors + cols[i], 1u)] = (uint32_t)i;
+}
+__global__ void transpose_sort_kernel(uint32_t width, const uint32_t* __restrict__ starts,
+                                      const uint32_t* __restrict__ entry_row, uint32_t* __restrict__ at,
+                                      uint32_t* __restrict__ rows) {
+  extern __shared__ uint32_t list[];
+  for (uint32_t c = blockIdx.x; c < width; c += gridDim.x) {
+    const uint32_t b = starts[c], n = starts[c + 1] - b;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) list[i] = at[b + i];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+      const uint32_t mine = list[i];
+      uint32_t place = 0;
+      for (uint32_t k = 0; k < n; ++k) place += list[k] < mine;
+      at[b + place] = mine;
+      rows[b + place] = entry_row[mine];
+    }
+    __syncthreads();
+  }
+}
+
 // One block of P = T - omega D^-1 A_f T (transfer.rs:108-152): A's blocks whose column is the row
 // or a smoothing neighbour act on that column's tentative block; the others are lumped onto the
 // row's own (src = row). Contributions to this block's coarse column add in A's column order.
@@ -1082,6 +1113,22 @@ sf_status setup_entry_rows(cudaStream_t st, uint32_t rows, const uint32_t* start
   if (rows == 0) return SF_OK;
   entry_rows_kernel<<<grid_for(rows), kT, 0, st>>>(rows, starts, out);
   return cuda_check(cudaGetLastError(), "entry rows");
+}
+
+sf_status setup_column_counts(cudaStream_t st, size_t entries, const uint32_t* cols, uint32_t* counts) {
+  if (entries == 0) return SF_OK;
+  column_counts_kernel<<<grid_for(entries), kT, 0, st>>>(entries, cols, counts);
+  return cuda_check(cudaGetLastError(), "column counts");
+}
+
+sf_status setup_transpose_pattern(cudaStream_t st, size_t entries, const uint32_t* cols, const uint32_t* entry_row,
+                                  uint32_t width, uint32_t longest, const uint32_t* t_starts, uint32_t* cursors,
+                                  uint32_t* t_at, uint32_t* t_rows) {
+  if (entries == 0) return SF_OK;
+  transpose_fill_kernel<<<grid_for(entries), kT, 0, st>>>(entries, cols, cursors, t_at);
+  transpose_sort_kernel<<<std::min<uint32_t>(width, 148 * 16), 128, longest * 4, st>>>(width, t_starts, entry_row, t_at,
+                                                                                       t_rows);
+  return cuda_check(cudaGetLastError(), "transpose pattern");
 }
 
 sf_status setup_rigid_modes(cudaStream_t st, uint32_t rows, const uint32_t* row_node, const double* nodes,

@@ -369,10 +369,10 @@ sf_status device_bsr(DeviceSolver& s, const Bsr& h, DevBsr& d, bool alias) {
   d.rows = (uint32_t)h.rows;
   d.rb = (uint32_t)h.rb;
   d.cb = (uint32_t)h.cb;
-  d.blocks = h.cols.size();
+  d.blocks = h.starts.back();
   d.starts = h.dev_starts;
   d.cols = h.dev_cols;
-  const size_t n = h.cols.size() * h.rb * h.cb;
+  const size_t n = d.blocks * h.rb * h.cb;
   if (alias && sizeof(S) == 8) {
     d.vals = h.dev;
   } else {
@@ -389,28 +389,6 @@ sf_status device_bsr(DeviceSolver& s, const Bsr& h, DevBsr& d, bool alias) {
     if (sf_status e = make_sell_converted<S>(s, d, h.starts.data(), h.cols.data(), h.dev)) return e;
   }
   return cuda_check(cudaGetLastError(), "level operator");
-}
-
-// The pattern of a prolongator's explicit transpose (coarse rows, fine block columns ascending)
-// and, per transposed block, the prolongator block it comes from (gpu/layout.rs:254-291 stores
-// the same transpose for gather restriction).
-void transpose_pattern(const Bsr& p, size_t coarse_rows, Bsr& t, std::vector<uint32_t>& src) {
-  t = Bsr();
-  t.rows = coarse_rows;
-  t.rb = p.cb;
-  t.cb = p.rb;
-  t.starts.assign(coarse_rows + 1, 0);
-  for (uint32_t c : p.cols) t.starts[c + 1] += 1;
-  for (size_t i = 0; i < coarse_rows; ++i) t.starts[i + 1] += t.starts[i];
-  std::vector<uint32_t> fill(t.starts.begin(), t.starts.end() - 1);
-  t.cols.resize(p.cols.size());
-  src.resize(p.cols.size());
-  for (size_t row = 0; row < p.rows; ++row)
-    for (uint32_t at = p.starts[row]; at < p.starts[row + 1]; ++at) {
-      uint32_t o = fill[p.cols[at]]++;
-      t.cols[o] = (uint32_t)row;
-      src[o] = at;
-    }
 }
 
 template <typename S>
@@ -432,22 +410,22 @@ sf_status upload_level(DeviceSolver& s, const std::vector<HostLevel>& levels, si
   L.has_p = h.has_p;
   if (h.has_p) {
     if (sf_status e = device_bsr<S>(s, h.p, L.p, alias)) return e;
+    // The explicit transpose (the reference's GPU layout stores the same one for gather restriction,
+    // gpu/layout.rs:254-291), its pattern as the Galerkin product made it.
     Bsr t;
-    std::vector<uint32_t> src;
-    transpose_pattern(h.p, levels[li + 1].a.rows, t, src);
-    uint32_t* d_src = nullptr;
-    sf_status e = dev_alloc(s, (void**)&d_src, std::max<size_t>(1, src.size()) * 4);
-    if (!e) e = dev_alloc(s, (void**)&t.dev_starts, (t.rows + 1) * 4);
-    if (!e) e = dev_alloc(s, (void**)&t.dev_cols, std::max<size_t>(1, t.cols.size()) * 4);
-    if (!e) e = dev_alloc(s, (void**)&t.dev, std::max<size_t>(1, t.cols.size()) * t.rb * t.cb * 8);
+    t.rows = levels[li + 1].a.rows;
+    t.rb = h.p.cb;
+    t.cb = h.p.rb;
+    t.starts = h.t_starts;
+    t.dev_starts = h.dev_t_starts;
+    t.dev_cols = h.dev_t_rows;
+    const size_t blocks = t.starts.back();
+    sf_status e = dev_alloc(s, (void**)&t.dev, std::max<size_t>(1, blocks) * t.rb * t.cb * 8);
     if (e) return e;
-    if (!src.empty()) copy_h2d(s, d_src, src.data(), src.size() * 4);
-    copy_h2d(s, t.dev_starts, t.starts.data(), (t.rows + 1) * 4);
-    if (!t.cols.empty()) copy_h2d(s, t.dev_cols, t.cols.data(), t.cols.size() * 4);
-    e = setup_transpose_blocks<double>(s.stream, t.cols.size(), (int)h.p.rb, (int)h.p.cb, d_src, h.p.dev, t.dev);
+    e = setup_transpose_blocks<double>(s.stream, blocks, (int)h.p.rb, (int)h.p.cb, h.dev_t_at, h.p.dev, t.dev);
     if (!e) e = device_bsr<S>(s, t, L.r, alias);
     if (!e) e = cuda_check(cudaStreamSynchronize(s.stream), "transpose");
-    dev_free(s, d_src);
+    dev_free(s, h.dev_t_at);
     if (sizeof(S) != 8) dev_free(s, t.dev);  // the converted copy is the one kept
     if (e) return e;
   }
