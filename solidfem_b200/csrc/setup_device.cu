@@ -240,43 +240,42 @@ __global__ void __launch_bounds__(kNormThreads) norm_sums_kernel(size_t n, uint3
   }
 }
 
-__global__ void __launch_bounds__(kNormThreads) norm_terms_kernel(size_t n, uint32_t chunks, const double* __restrict__ x,
-                                                                  const int* __restrict__ binades, Increment* pairs,
-                                                                  unsigned* ticket, double* __restrict__ norm) {
+// Chunk c's pair for the binade e, in lane 0 of the warp that makes it.
+__device__ __forceinline__ Increment chunk_increment(size_t n, uint32_t c, const double* __restrict__ x, int e) {
   constexpr int kPer = kNormChunk / 32;
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t c = blockIdx.x * (kNormThreads / 32) + warp;
-  if (c < chunks && binades[c] != kNoBinade) {
-    const double scale = __longlong_as_double((long long)(52 - binades[c] + 1023) << 52);  // 1 / u
-    Increment t = {0, 0};
+  const uint32_t lane = threadIdx.x & 31;
+  const double scale = __longlong_as_double((long long)(52 - e + 1023) << 52);  // 1 / u
+  Increment t = {0, 0};
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      const size_t i = (size_t)c * kNormChunk + lane * kPer + k;
-      const double v = i < n ? x[i] : 0.0;
-      // y / u exactly (a result below one half may round, and stays below one half); a term past
-      // the binade's end is held at 2^53, which no s in the binade survives.
-      const double q = fmin(v * v * scale, 9007199254740992.0), whole = floor(q), part = q - whole;
-      const unsigned long long m = (unsigned long long)whole;
-      Increment one;
-      one.even = m + (part > 0.5 || (part == 0.5 && (m & 1)) ? 1 : 0);
-      one.odd = m + (part > 0.5 || (part == 0.5 && !(m & 1)) ? 1 : 0);
-      t = then(t, one);
-    }
-    for (int o = 1; o < 32; o <<= 1) {
-      Increment r;
-      r.even = __shfl_down_sync(0xffffffffu, t.even, o);
-      r.odd = __shfl_down_sync(0xffffffffu, t.odd, o);
-      t = then(t, r);
-    }
-    if (lane == 0) {
-      t.even = min(t.even, 1ull << 53);
-      t.odd = min(t.odd, 1ull << 53);
-      __stcg(&pairs[c].even, t.even);
-      __stcg(&pairs[c].odd, t.odd);
-    }
+  for (int k = 0; k < kPer; ++k) {
+    const size_t i = (size_t)c * kNormChunk + lane * kPer + k;
+    const double v = i < n ? x[i] : 0.0;
+    // y / u exactly (a result below one half may round, and stays below one half); a term past
+    // the binade's end is held at 2^53, which no s in the binade survives.
+    const double q = fmin(v * v * scale, 9007199254740992.0), whole = floor(q), part = q - whole;
+    const unsigned long long m = (unsigned long long)whole;
+    Increment one;
+    one.even = m + (part > 0.5 || (part == 0.5 && (m & 1)) ? 1 : 0);
+    one.odd = m + (part > 0.5 || (part == 0.5 && !(m & 1)) ? 1 : 0);
+    t = then(t, one);
   }
-  if (!last_block(ticket) || warp != 0) return;
-  __shared__ double y[kNormChunk];
+  for (int o = 1; o < 32; o <<= 1) {
+    Increment r;
+    r.even = __shfl_down_sync(0xffffffffu, t.even, o);
+    r.odd = __shfl_down_sync(0xffffffffu, t.odd, o);
+    t = then(t, r);
+  }
+  t.even = min(t.even, 1ull << 53);
+  t.odd = min(t.odd, 1ull << 53);
+  return t;
+}
+
+// The walk over the chunks by one warp; y is its buffer of kNormChunk terms. Every lane returns s.
+template <class Binade, class Pair>
+__device__ __forceinline__ double norm_walk(size_t n, uint32_t chunks, const double* __restrict__ x, double* y,
+                                            Binade&& binade_of, Pair&& pair_of) {
+  constexpr int kPer = kNormChunk / 32;
+  const uint32_t lane = threadIdx.x & 31;
   double s = 0.0;  // the same in every lane
   // s after the increment `t`, when it stays in its binade
   auto advance = [&](const Increment& t) {
@@ -292,11 +291,8 @@ __global__ void __launch_bounds__(kNormThreads) norm_terms_kernel(size_t n, uint
     int e = kNoBinade;
     Increment p = {0, 0};
     if (mine < chunks) {
-      e = __ldg(binades + mine);
-      if (e != kNoBinade) {
-        p.even = __ldcg(&pairs[mine].even);
-        p.odd = __ldcg(&pairs[mine].odd);
-      }
+      e = binade_of(mine);
+      if (e != kNoBinade) p = pair_of(mine);
     }
     const int now = binade(s);
     if (now != kNoBinade && __all_sync(0xffffffffu, mine >= chunks || e == now)) {
@@ -329,7 +325,77 @@ __global__ void __launch_bounds__(kNormThreads) norm_terms_kernel(size_t n, uint
       for (int i = 0; i < kNormChunk; ++i) s += y[i];
     }
   }
+  return s;
+}
+
+__global__ void __launch_bounds__(kNormThreads) norm_terms_kernel(size_t n, uint32_t chunks, const double* __restrict__ x,
+                                                                  const int* __restrict__ binades, Increment* pairs,
+                                                                  unsigned* ticket, double* __restrict__ norm) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t c = blockIdx.x * (kNormThreads / 32) + warp;
+  if (c < chunks && binades[c] != kNoBinade) {
+    const Increment t = chunk_increment(n, c, x, binades[c]);
+    if (lane == 0) {
+      __stcg(&pairs[c].even, t.even);
+      __stcg(&pairs[c].odd, t.odd);
+    }
+  }
+  if (!last_block(ticket) || warp != 0) return;
+  __shared__ double y[kNormChunk];
+  const double s = norm_walk(
+      n, chunks, x, y, [&](uint32_t k) { return __ldg(binades + k); },
+      [&](uint32_t k) {
+        Increment p;
+        p.even = __ldcg(&pairs[k].even);
+        p.odd = __ldcg(&pairs[k].odd);
+        return p;
+      });
   if (lane == 0) *norm = sqrt(s);
+}
+
+// The norm and v = x / norm of a small vector in one block, a chunk to a warp: the three launches of
+// a large one cost more than their work (a level of 318 unknowns: its 20 power iterations
+// 0.69 -> 0.55 ms).
+constexpr uint32_t kSmallChunks = 32;
+__global__ void __launch_bounds__(32 * kSmallChunks) small_normalize_kernel(size_t n, uint32_t chunks,
+                                                                            const double* __restrict__ x,
+                                                                            double* __restrict__ norm,
+                                                                            double* __restrict__ v) {
+  __shared__ double sums[kSmallChunks], y[kNormChunk], length;
+  __shared__ int binades[kSmallChunks];
+  __shared__ Increment pairs[kSmallChunks];
+  const uint32_t lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+  double s = 0.0;
+  if (c < chunks)
+#pragma unroll
+    for (int k = 0; k < kNormChunk / 32; ++k) {
+      const size_t i = (size_t)c * kNormChunk + 32 * k + lane;
+      const double w = i < n ? x[i] : 0.0;
+      s += w * w;
+    }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) sums[c] = s;
+  __syncthreads();
+  if (c < chunks) {
+    double before = 0.0;
+    for (uint32_t k = 0; k < c; ++k) before += sums[k];
+    const int e = binade(before), use = e == binade(before + sums[c]) ? e : kNoBinade;
+    Increment t = {0, 0};
+    if (use != kNoBinade) t = chunk_increment(n, c, x, use);
+    if (lane == 0) {
+      binades[c] = use;
+      pairs[c] = t;
+    }
+  }
+  __syncthreads();
+  if (c == 0) {
+    const double total = norm_walk(
+        n, chunks, x, y, [&](uint32_t k) { return binades[k]; }, [&](uint32_t k) { return pairs[k]; });
+    if (lane == 0) *norm = length = sqrt(total);
+  }
+  __syncthreads();
+  const double by = length;
+  for (size_t i = threadIdx.x; i < n; i += blockDim.x) v[i] = x[i] / by;
 }
 
 // s2 = D^-1 (A v) for one block row per thread, in the order of setup.rs:404-432.
@@ -539,9 +605,12 @@ __global__ void product_kernel(size_t entries, const uint32_t* __restrict__ entr
   }
 }
 
-// One block of P^T (A P) (transfer.rs:173-238): the fine rows of P's column in ascending order,
-// each P block transposed times the A P block of that fine row at this block's column; a zero on
-// the diagonal of a diagonal block becomes one (finish_level, setup.rs:650-695).
+// One row of a block of P^T (A P) per thread (transfer.rs:173-238): the fine rows of P's column in
+// ascending order, row r of each P block transposed times the A P block of that fine row at this
+// block's column; a zero on the diagonal of a diagonal block becomes one (finish_level,
+// setup.rs:650-695). A coarse row sums tens to hundreds of fine rows and a small level has few
+// blocks, so the chain of one thread bounds it: six threads a block instead of one, each of the same
+// terms in the same order (817 blocks of about 170 fine rows: the phase 0.72 -> 0.49 ms).
 template <int N>
 __global__ void galerkin_kernel(size_t entries, const uint32_t* __restrict__ entry_row, const uint32_t* __restrict__ c_cols,
                                 const uint32_t* __restrict__ pt_starts, const uint32_t* __restrict__ pt_rows,
@@ -549,11 +618,13 @@ __global__ void galerkin_kernel(size_t entries, const uint32_t* __restrict__ ent
                                 const uint32_t* __restrict__ ap_starts, const uint32_t* __restrict__ ap_cols,
                                 const double* __restrict__ ap_vals, double* __restrict__ c_vals) {
   constexpr int L = N * 6;
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < entries; j += (size_t)gridDim.x * blockDim.x) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < 6 * entries; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t j = i / 6;
+    const int r = (int)(i % 6);
     const uint32_t crow = entry_row[j], c = c_cols[j];
-    double acc[36];
+    double acc[6];
 #pragma unroll
-    for (int i = 0; i < 36; ++i) acc[i] = 0.0;
+    for (int q = 0; q < 6; ++q) acc[q] = 0.0;
     for (uint32_t k = pt_starts[crow]; k < pt_starts[crow + 1]; ++k) {
       const uint32_t fine_row = pt_rows[k];
       const uint32_t* b = ap_cols + ap_starts[fine_row];
@@ -568,24 +639,22 @@ __global__ void galerkin_kernel(size_t entries, const uint32_t* __restrict__ ent
           hi = mid;
       }
       if (lo == e || *lo != c) continue;
-      const double* pb = p_vals + (size_t)pt_at[k] * L;
+      const double* pb = p_vals + (size_t)pt_at[k] * L + r;
       const double* ab = ap_vals + (size_t)(lo - ap_cols) * L;
 #pragma unroll
-      for (int r = 0; r < 6; ++r)
+      for (int m = 0; m < N; ++m) {
+        double s = pb[m * 6];
 #pragma unroll
-        for (int m = 0; m < N; ++m) {
-          double s = pb[m * 6 + r];
-#pragma unroll
-          for (int q = 0; q < 6; ++q) acc[r * 6 + q] += s * ab[m * 6 + q];
-        }
+        for (int q = 0; q < 6; ++q) acc[q] += s * ab[m * 6 + q];
+      }
     }
     if (crow == c)
 #pragma unroll
-      for (int d = 0; d < 6; ++d)
-        if (acc[d * 6 + d] == 0.0) acc[d * 6 + d] = 1.0;
-    double* out = c_vals + j * 36;
+      for (int q = 0; q < 6; ++q)
+        if (q == r && acc[q] == 0.0) acc[q] = 1.0;
+    double* out = c_vals + j * 36 + r * 6;
 #pragma unroll
-    for (int i = 0; i < 36; ++i) out[i] = acc[i];
+    for (int q = 0; q < 6; ++q) out[q] = acc[q];
   }
 }
 
@@ -1035,6 +1104,10 @@ sf_status setup_start_vector(cudaStream_t st, size_t n, double* v) {
 sf_status setup_normalize(cudaStream_t st, size_t n, const double* src, void* scratch, double* norm, double* v) {
   if (n == 0) return SF_OK;
   const uint32_t chunks = (uint32_t)((n + kNormChunk - 1) / kNormChunk);
+  if (chunks <= kSmallChunks) {
+    small_normalize_kernel<<<1, 32 * kSmallChunks, 0, st>>>(n, chunks, src, norm, v);
+    return cuda_check(cudaGetLastError(), "normalize");
+  }
   unsigned* tickets = (unsigned*)scratch;
   Increment* pairs = (Increment*)((char*)scratch + 256);
   double* sums = (double*)(pairs + chunks);
@@ -1210,10 +1283,10 @@ sf_status setup_galerkin(cudaStream_t st, int rb, size_t entries, const uint32_t
                          const uint32_t* ap_starts, const uint32_t* ap_cols, const double* ap_vals, double* c_vals) {
   if (entries == 0) return SF_OK;
   if (rb == 3)
-    galerkin_kernel<3><<<grid_for(entries), kT, 0, st>>>(entries, entry_row, c_cols, pt_starts, pt_rows, pt_at, p_vals,
+    galerkin_kernel<3><<<grid_for(6 * entries), kT, 0, st>>>(entries, entry_row, c_cols, pt_starts, pt_rows, pt_at, p_vals,
                                                          ap_starts, ap_cols, ap_vals, c_vals);
   else
-    galerkin_kernel<6><<<grid_for(entries), kT, 0, st>>>(entries, entry_row, c_cols, pt_starts, pt_rows, pt_at, p_vals,
+    galerkin_kernel<6><<<grid_for(6 * entries), kT, 0, st>>>(entries, entry_row, c_cols, pt_starts, pt_rows, pt_at, p_vals,
                                                          ap_starts, ap_cols, ap_vals, c_vals);
   return cuda_check(cudaGetLastError(), "galerkin");
 }
