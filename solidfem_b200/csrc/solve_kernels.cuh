@@ -2179,7 +2179,7 @@ __device__ __forceinline__ void jacobi_update_p_kernel(uint32_t n, const double*
 
 // The update's 592 blocks are four to an SM: at 64 registers they run as one wave (left to itself it
 // takes 122, two blocks to an SM and two waves): 603,000 unknowns in f64 727 -> 714 us an iteration,
-// in mixed precision 465 -> 460, 45^3 cells under Jacobi 33 -> 31.
+// 45^3 cells under Jacobi 33 -> 31, mixed precision unchanged.
 template <>
 struct Resident<pcg_update_kernel> {
   static constexpr int blocks = 4;
