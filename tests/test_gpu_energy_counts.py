@@ -1,5 +1,5 @@
-"""sf_study_energy_products over every vector count on SELL systems, whose kernel is chosen by the
-count: one vector, up to four in one group, five to eight in two groups (needs a B200)."""
+"""sf_study_energy_products over every vector count on SELL and row-group systems, whose kernels are
+chosen by the count: one vector, up to four in one walk, five to eight in two (needs a B200)."""
 import numpy as np
 import pytest
 
@@ -11,10 +11,11 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("count", range(1, 9))
-@pytest.mark.parametrize("div", [(1, 1, 1), (12, 3, 3)])  # under one slice; a ragged last slice
-def test_every_count(div, count):
+@pytest.mark.parametrize("sell", [1, 0])
+@pytest.mark.parametrize("div", [(1, 1, 1), (12, 3, 3), (30, 7, 6)])  # under one slice or block; ragged last ones
+def test_every_count(div, sell, count):
     _, model = product_model((10.0, 1.0, 1.0), div, 200000.0, 0.3)
-    study = sf.StaticStudy.new(model, mg_options(sf.Precision.DOUBLE, sell_min_rows=1))
+    study = sf.StaticStudy.new(model, mg_options(sf.Precision.DOUBLE, sell_min_rows=sell))
     xs = np.random.default_rng(count).standard_normal((count, study.report()["free_dofs"]))
     check_against_system_multiply(study, xs, *energy_products(study, xs))
 
