@@ -808,7 +808,8 @@ sf_status solver_read_state(DeviceSolver& s, PcgState* out) {
 // A variant of the conjugate gradient's system product (pcg_spmv_dot_kernel and
 // sell_pcg_spmv_dot_kernel): for each of `count` vectors x_k of caller-owned device memory it
 // writes y_k = A x_k and the energy e_k = x_k . y_k. Rows are summed exactly as the system product
-// sums them; up to four vectors go through one walk of the operator, five to eight through two. The reduction's scratch is not the solver's: it is
+// sums them; up to four vectors go through one walk of the operator, five to eight through two.
+// The reduction's scratch is not the solver's: it is
 // the file-scope array below, whose address is looked up once per device, so a call allocates no
 // memory at all.
 //
