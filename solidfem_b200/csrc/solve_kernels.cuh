@@ -49,8 +49,8 @@ const int kSmemPerBlockTarget = 72 * 1024;
 // Without a programmatic predecessor the wait returns at once.
 // Only the row-group engine and the coarse solve release their successors early, and the vector
 // kernels at sizes of one element a thread: 16 cantilevers in a batch 17.1 -> 13.1 ms, one of 9,720
-// unknowns 76 -> 70 us an iteration. The SELL and split-row walks do not: their registers went from
-// 109 to 126 and more with the first chunk before the wait, and 603,000 unknowns from 472 to 488 us.
+// unknowns 76 -> 70 us an iteration. The SELL and split-row walks do not: with the first chunk held
+// across the wait their registers went from 109 to 126 and more, and with them resident warps.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 constexpr uint32_t kOneWave = kReduceBlocks * kReduceThreads;  // unknowns the vector kernels take one per thread
 constexpr uint32_t kOneWaveRows = kOneWave / 3;
