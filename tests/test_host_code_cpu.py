@@ -1,0 +1,35 @@
+"""Host code of the library on a stand-in CUDA runtime (tests/native/fake_cuda.h), whose calls can be
+told to fail: no device is needed, and none is asked to fail."""
+import os
+import subprocess
+
+import pytest
+
+from solidfem_b200 import build as b
+
+NATIVE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "native")
+
+
+def program(folder, name):
+    """tests/native/<name>.cpp with the library's <name>.cpp."""
+    out = str(folder / name)
+    subprocess.run([b.CXX, "-std=c++17", "-O1", "-fopenmp", "-Wno-unused-function", "-I" + NATIVE, "-I" + b.CSRC,
+                    "-I" + os.path.join(b.CUDA, "include"), os.path.join(NATIVE, name + ".cpp"),
+                    os.path.join(b.CSRC, name + ".cpp"), "-o", out], check=True, capture_output=True, text=True)
+    return out
+
+
+def run(*command):
+    r = subprocess.run([str(c) for c in command], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.fixture(scope="module")
+def host_link(tmp_path_factory):
+    return program(tmp_path_factory.mktemp("host_link"), "host_link")
+
+
+@pytest.mark.parametrize("pinned", ["pinned", "no-pinned", "one-pinned"])
+@pytest.mark.parametrize("size", [0, 8, (64 << 10) - 8, 64 << 10, (4 << 20) + 8, 9 << 20])
+def test_arrays_cross_whether_or_not_page_locked_memory_is_to_be_had(host_link, pinned, size):
+    run(host_link, pinned, size)
