@@ -34,6 +34,20 @@ void round_trip(size_t n, int pinned) {
   CHECK(cudaGetLastError() == cudaSuccess);  // a refused allocation is nobody else's error
 }
 
+// The caller's array may be reused once copy_in has returned, page-locked or not.
+void reuse(size_t n) {
+  DeviceSolver d;
+  void* src = nullptr;
+  CHECK(cudaMallocHost(&src, n) == cudaSuccess);
+  const std::vector<char> first = pattern(n);
+  std::memcpy(src, first.data(), n);
+  std::vector<char> device(n), keep(n);
+  CHECK(copy_in(d, device.data(), src, keep.data(), n, 3) == SF_OK);
+  std::memset(src, 0xff, n);
+  fake::drain();
+  CHECK(device == first && keep == first);
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -42,5 +56,6 @@ int main(int argc, char** argv) {
   if (what == "pinned") round_trip(n, 1 << 30);
   if (what == "no-pinned") round_trip(n, 0);
   if (what == "one-pinned") round_trip(n, 1);
+  if (what == "reuse") reuse(n);
   return 0;
 }

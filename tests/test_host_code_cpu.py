@@ -33,3 +33,8 @@ def host_link(tmp_path_factory):
 @pytest.mark.parametrize("size", [0, 8, (64 << 10) - 8, 64 << 10, (4 << 20) + 8, 9 << 20])
 def test_arrays_cross_whether_or_not_page_locked_memory_is_to_be_had(host_link, pinned, size):
     run(host_link, pinned, size)
+
+
+@pytest.mark.parametrize("size", [8, (64 << 10) - 8, 64 << 10, 9 << 20])
+def test_a_load_vector_may_be_reused_once_it_was_taken(host_link, size):
+    run(host_link, "reuse", size)
