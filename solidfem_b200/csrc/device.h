@@ -151,6 +151,7 @@ struct DeviceSolver {
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraph_t run_graph = nullptr;           // kRunIterations iterations in one graph
   cudaGraphExec_t run_exec = nullptr;
+  bool run_failed = false;                   // it could not be made
   uint64_t iterations_run = 0;               // by this solver, over all its solves
   uint64_t launches_per_iteration = 0;
   uint64_t graph_kernels = 0;     // kernel nodes in the captured iteration graph
@@ -383,7 +384,6 @@ sf_status solver_level_stage(DeviceSolver& s, size_t level, int stage, const dou
 sf_status solver_precondition(DeviceSolver& s, const double* d_in, double* d_out);
 sf_status solver_system_multiply(DeviceSolver& s, const double* d_in, double* d_out);
 sf_status solver_capture_graph(DeviceSolver& s);
-sf_status solver_capture_run(DeviceSolver& s);  // kRunIterations iterations
 sf_status solver_read_state(DeviceSolver& s, PcgState* out);
 // Pcg::step on the device (study.cpp): up to max_iterations iterations replayed in chunks with one
 // state read-back per chunk into `pinned`; updates last, status and cancelled.

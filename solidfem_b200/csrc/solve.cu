@@ -488,35 +488,6 @@ sf_status solver_enqueue_iteration(DeviceSolver& s) {
   return solver_enqueue_reset(s);
 }
 
-namespace {
-sf_status capture_iterations(DeviceSolver& s, uint64_t count, cudaGraph_t* graph, cudaGraphExec_t* exec) {
-  cudaError_t e = cudaStreamBeginCapture(s.stream, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) return cuda_check(e, "begin capture");
-  sf_status st = SF_OK;
-  for (uint64_t i = 0; i < count && !st; ++i) st = solver_enqueue_iteration(s);
-  cudaGraph_t g = nullptr;
-  e = cudaStreamEndCapture(s.stream, &g);
-  *graph = g;
-  if (st) return st;
-  if (e != cudaSuccess) return cuda_check(e, "end capture");
-  return cuda_check(cudaGraphInstantiate(exec, g, 0), "graph instantiate");
-}
-}  // namespace
-
-sf_status solver_capture_graph(DeviceSolver& s) {
-  if (s.graph_exec) return SF_OK;
-  if (sf_status e = capture_iterations(s, 1, &s.graph, &s.graph_exec)) return e;
-  size_t nodes = 0;
-  cudaGraphGetNodes(s.graph, nullptr, &nodes);
-  s.graph_kernels = nodes;
-  return SF_OK;
-}
-
-sf_status solver_capture_run(DeviceSolver& s) {
-  if (s.run_exec) return SF_OK;
-  return capture_iterations(s, kRunIterations, &s.run_graph, &s.run_exec);
-}
-
 // ------------------------------------------------------------ batched iterations
 // Records one conjugate gradient iteration of every instance, checks that they launch the same
 // kernels in the same order with the same block shapes, and captures one graph whose every node

@@ -1328,56 +1328,6 @@ static void fill_progress(const PcgState& st, sf_progress* p) {
 
 namespace sf {
 
-// Pcg::step (pcg.rs:167-190) on the device: up to max_iterations iterations, enqueued in chunks;
-// every kernel of an iteration after the solve ends returns at once, so the state is read back
-// once per chunk, with one chunk in flight ahead. `cancel` is read before every iteration.
-sf_status run_iterations(DeviceSolver& d, bool use_graphs, uint64_t max_iterations, sf_cancel_fn cancel, void* user,
-                         PcgState* pinned, PcgState& last, int& status, bool& cancelled) {
-  uint64_t done = 0;
-  const uint64_t chunk_max = 16;
-  uint64_t chunk = 4;
-  bool stop = false;
-  while (!stop && done < max_iterations) {
-    uint64_t k = std::min<uint64_t>(chunk, max_iterations - done);
-    uint64_t launched = 0;
-    while (launched < k) {
-      // Whole runs of iterations where no cancel must be read between them.
-      if (use_graphs && !cancel && k - launched >= kRunIterations && d.n <= kRunMaxUnknowns &&
-          d.iterations_run >= kRunAfter) {
-        if (sf_status e = solver_capture_run(d)) return e;
-        if (sf_status e = cuda_check(cudaGraphLaunch(d.run_exec, d.stream), "graph launch")) return e;
-        d.launches += kRunIterations * d.graph_kernels;
-        launched += kRunIterations;
-        continue;
-      }
-      if (cancel && cancel(user)) {
-        cancelled = true;
-        stop = true;
-        break;
-      }
-      sf_status e = SF_OK;
-      if (use_graphs) {
-        e = cuda_check(cudaGraphLaunch(d.graph_exec, d.stream), "graph launch");
-        d.launches += d.graph_kernels;
-      } else {
-        e = solver_enqueue_iteration(d);
-        d.launches += d.launches_per_iteration;
-      }
-      if (e) return e;
-      ++launched;
-    }
-    done += launched;
-    d.iterations_run += launched;
-    copy_d2h(d, pinned, d.state, sizeof(PcgState));
-    if (sf_status e = cuda_check(cudaStreamSynchronize(d.stream), "solver step")) return e;
-    last = *pinned;
-    status = last.status;
-    if (status != ST_ACTIVE) stop = true;
-    chunk = std::min(chunk_max, chunk * 2);
-  }
-  return SF_OK;
-}
-
 // The StepOutcome of a step that ended with `status` (pcg.rs:47-57, 216-275): the kind and the
 // progress, and for a failed solve its PcgError as the returned status with its payload.
 sf_status step_result(int status, bool cancelled, const PcgState& last, sf_step_outcome* out) {

@@ -38,3 +38,13 @@ def test_arrays_cross_whether_or_not_page_locked_memory_is_to_be_had(host_link, 
 @pytest.mark.parametrize("size", [8, (64 << 10) - 8, 64 << 10, 9 << 20])
 def test_a_load_vector_may_be_reused_once_it_was_taken(host_link, size):
     run(host_link, "reuse", size)
+
+
+@pytest.fixture(scope="module")
+def iterations(tmp_path_factory):
+    return program(tmp_path_factory.mktemp("iterations"), "iterations")
+
+
+@pytest.mark.parametrize("case", ["whole", "no-instantiation", "no-capture", "no-launch"])
+def test_a_solve_does_not_need_its_longer_graph(iterations, case):
+    run(iterations, case)
