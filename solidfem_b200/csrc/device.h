@@ -101,12 +101,14 @@ struct PcgState {
 };
 
 // Iterations in the longer graph of a small solver. Between two graphs the last kernel must finish
-// and the next graph start, 6 us in which nothing runs, where kernels of one graph follow each other
-// by programmatic launches: 69.8 -> 64.0 us an iteration at 9,720 unknowns, no difference at 217,800
-// (345 us an iteration). Its capture costs as much as a few dozen of those gaps, so it is made once a
-// solver has run kRunAfter iterations.
+// and the next graph start, where kernels of one graph follow each other by programmatic launches: a
+// step of 39 iterations at 9,720 unknowns 2,475 -> 2,415 us, at 130,000 unknowns 8,080 -> 7,980; raw
+// systems under Jacobi 30.0 -> 28.1 us an iteration at 91,125 unknowns; no difference at 217,800 (345
+// us an iteration). That is about 2 us an iteration, and the graph costs 130 us to make and upload with
+// Jacobi's 5 kernels an iteration, 280 to 470 us with multigrid's 14 to 28: it pays for itself after
+// about 16 iterations for each kernel, and is made when so many are in sight (iterations.cpp).
 static const uint64_t kRunIterations = 4;
-static const uint64_t kRunAfter = 64;
+static const uint64_t kRunWorthPerKernel = 16;
 static const uint32_t kRunMaxUnknowns = 151552;
 // Reduction scratch: one partial per block of the fixed reduction grid.
 static const int kReduceBlocks = 592;  // 4 x 148 SMs

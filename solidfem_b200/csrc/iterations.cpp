@@ -1,6 +1,7 @@
 // The solve's iterations as CUDA graphs, and the loop that replays them (host code; the kernels an
 // iteration enqueues are solve.cu's).
 #include <algorithm>
+#include <cmath>
 
 #include "device.h"
 
@@ -38,10 +39,22 @@ void give_up_run(DeviceSolver& s) {
   cudaGetLastError();
 }
 
-// Enqueues kRunIterations iterations as one graph; false when that is not to be had.
-bool launch_run(DeviceSolver& s) {
+// Iterations still to come by the mean rate of the `last` ones (0 while that says little), at most
+// `most`.
+uint64_t expected_iterations(const PcgState& last, uint64_t most) {
+  if (last.iterations < 12 || !(last.rel > last.tolerance && last.rel < 1.0) || !(last.tolerance > 0.0)) return 0;
+  const double more = (double)last.iterations * std::log(last.rel / last.tolerance) / -std::log(last.rel);
+  return more >= (double)most ? most : (uint64_t)more;
+}
+
+// Enqueues kRunIterations iterations as one graph; false when that is not to be had, or not worth
+// its making yet: `expected` more iterations are in sight, or `opening` a step, when what the solver
+// has run so far stands for what is to come.
+bool launch_run(DeviceSolver& s, bool opening, uint64_t expected) {
   if (s.run_failed) return false;
   if (!s.run_exec) {
+    const uint64_t worth = kRunWorthPerKernel * s.graph_kernels;
+    if (expected < worth && !(opening && s.iterations_run >= worth)) return false;
     const sf_error kept = error_slot();  // a failure here is not the caller's
     if (capture_iterations(s, kRunIterations, &s.run_graph, &s.run_exec)) {
       error_slot() = kept;
@@ -83,7 +96,7 @@ sf_status run_iterations(DeviceSolver& d, bool use_graphs, uint64_t max_iteratio
     while (launched < k) {
       // Whole runs of iterations where no cancel must be read between them.
       if (use_graphs && !cancel && k - launched >= kRunIterations && d.n <= kRunMaxUnknowns &&
-          d.iterations_run >= kRunAfter && launch_run(d)) {
+          launch_run(d, done == 0, done ? expected_iterations(last, max_iterations - done) : 0)) {
         launched += kRunIterations;
         continue;
       }

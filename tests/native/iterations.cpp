@@ -2,6 +2,8 @@
 // iteration counts itself in the solver's state.
 #include "fake_cuda.h"
 
+#include <cmath>
+
 #include "device.h"
 
 using namespace sf;
@@ -14,15 +16,17 @@ struct FakeGraph {
 FakeGraph* capturing = nullptr;
 int graphs = 0, execs = 0;  // alive
 int begins = 0;             // captures begun
+uint64_t kernels = 5;       // an iteration's
 int instantiations_left = 1 << 30, run_launches_left = 1 << 30, enqueues_left = 1 << 30;
 uint64_t run_launches = 0, single_launches = 0;
 PcgState* device_state = nullptr;
-uint64_t converges_at = ~0ull;
+uint64_t converges_at = 400;
 
 void iterate() {
   PcgState& s = *device_state;
   if (s.status != ST_ACTIVE) return;
   s.iterations += 1;
+  s.rel = std::pow(s.tolerance, (double)s.iterations / (double)converges_at);
   if (s.iterations >= converges_at) s.status = ST_CONVERGED;
 }
 
@@ -47,7 +51,7 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t g, unsigned lon
   return cudaSuccess;
 }
 cudaError_t cudaGraphGetNodes(cudaGraph_t g, cudaGraphNode_t*, size_t* n) {
-  *n = 5 * ((FakeGraph*)g)->iterations;
+  *n = kernels * ((FakeGraph*)g)->iterations;
   return cudaSuccess;
 }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
@@ -75,7 +79,7 @@ sf_error& error_slot() {
   return e;
 }
 sf_status solver_enqueue_iteration(DeviceSolver& s) {
-  s.launches_per_iteration = 5;
+  s.launches_per_iteration = kernels;
   if (enqueues_left-- <= 0) return SF_CUDA_ERROR;
   if (capturing)
     capturing->iterations += 1;
@@ -95,7 +99,8 @@ struct Solve {
   Solve() {
     d.n = 9720;
     d.state = device_state = &state;
-    CHECK(solver_capture_graph(d) == SF_OK && d.graph_kernels == 5);
+    state.tolerance = 1e-9;
+    CHECK(solver_capture_graph(d) == SF_OK && d.graph_kernels == kernels);
   }
   ~Solve() {  // as dev_free_all
     if (d.graph_exec) cudaGraphExecDestroy(d.graph_exec);
@@ -123,6 +128,32 @@ void no_run_graph() {
   CHECK(graphs == 0 && execs == 0);
 }
 
+// One solve of a new solver: whether the longer graph is made, and how many iterations it takes on.
+void one_solve(uint64_t iterations, bool made) {
+  converges_at = iterations;
+  Solve s;
+  CHECK(s.run(~0ull >> 1) == SF_OK && s.status == ST_CONVERGED && s.last.iterations == iterations);
+  CHECK(begins == (made ? 2 : 1));
+  CHECK(!made || kRunIterations * run_launches >= iterations - 2 * kRunWorthPerKernel);
+}
+
+// Short solves of a solver that stays: made at the start of one, once they add up.
+void many_solves(uint64_t iterations) {
+  converges_at = iterations;
+  Solve s;
+  for (uint64_t ran = 0, i = 0; i < 20; ++i) {
+    const bool due = ran >= kRunWorthPerKernel * kernels;
+    s.state.iterations = 0;
+    s.state.status = s.status = ST_ACTIVE;
+    s.state.rel = 1.0;
+    const uint64_t before = run_launches;
+    CHECK(s.run(~0ull >> 1) == SF_OK && s.last.iterations == iterations);
+    CHECK(begins == (due ? 2 : 1) && (run_launches > before) == due);
+    ran = s.d.iterations_run;
+  }
+  CHECK(begins == 2);
+}
+
 void whole_solve(uint64_t total) {
   {
     Solve s;
@@ -139,6 +170,13 @@ void whole_solve(uint64_t total) {
 int main(int argc, char** argv) {
   const std::string what = argv[1];
   if (what == "whole") whole_solve(203);
+  if (what == "soon-over") one_solve(90, false);
+  if (what == "long-enough") one_solve(100, true);
+  if (what == "long") one_solve(211, true);
+  if (what == "short-solves") {
+    kernels = 14;
+    many_solves(39);
+  }
   if (what == "no-instantiation") {
     instantiations_left = 1;
     no_run_graph();

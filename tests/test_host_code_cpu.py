@@ -48,3 +48,11 @@ def iterations(tmp_path_factory):
 @pytest.mark.parametrize("case", ["whole", "no-instantiation", "no-capture", "no-launch"])
 def test_a_solve_does_not_need_its_longer_graph(iterations, case):
     run(iterations, case)
+
+
+@pytest.mark.parametrize("case", ["soon-over", "long-enough", "long", "short-solves"])
+def test_the_longer_graph_is_made_where_it_pays(iterations, case):
+    """5 kernels an iteration: worth 80 iterations. Looked at from iteration 12 on, a solve of 90 has 78
+    to go and does not make it, solves of 100 and 211 do. 14 kernels: worth 224, the sixth solve of 39
+    has seen 195, the seventh more."""
+    run(iterations, case)
