@@ -977,42 +977,97 @@ __global__ void split_fill_kernel(size_t slots, const uint32_t* __restrict__ sel
   }
 }
 
-// A thread per block row merges its three scalar rows: the next block column is the least of the
-// rows' next columns over three (and, for the padded last block row, its own diagonal block).
+// How many of the lanes' `block`s (ascending, a lane each) are below `key`.
+__device__ __forceinline__ uint32_t lanes_below(uint32_t block, uint32_t key) {
+  uint32_t at = 0;
+#pragma unroll
+  for (uint32_t step = 16; step > 0; step >>= 1)
+    if (__shfl_sync(0xffffffffu, block, at + step - 1) < key) at += step;
+  return at + (__shfl_sync(0xffffffffu, block, at) < key);
+}
+
+// A warp per block row merges its three scalar rows (and, for the padded last block row, its own
+// diagonal block), 32 entries of each at a time: what lies below the first block column that may go
+// on past a row's 32 is taken. A block's place is the number of first entries of smaller blocks, a
+// first entry being a block's first in its row where no row before it has the block. Columns are
+// strictly ascending, so a block has three entries of a row at most and every step takes 29 or more
+// of some row. A thread per block row read a dense row as one chain of loads: 91,125 unknowns with
+// one full row and column were created in 48 ms.
 __global__ void padded_blocks_kernel(uint64_t n, uint32_t rows, const uint64_t* __restrict__ rs,
                                      const uint32_t* __restrict__ cols, const double* __restrict__ scalars,
                                      const uint32_t* __restrict__ out_starts, uint32_t* __restrict__ out,
                                      double* __restrict__ vals) {
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr uint32_t kNone = 0xffffffffu;  // past a row's end
+  const uint32_t lane = threadIdx.x & 31, b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (b >= rows) return;
   uint64_t at[3], end[3];
+#pragma unroll
   for (int p = 0; p < 3; ++p) {
     const uint64_t r = 3 * (uint64_t)b + p;
     at[p] = r < n ? rs[r] : 0;
     end[p] = r < n ? rs[r + 1] : 0;
   }
   bool own = 3 * (uint64_t)b + 3 > n;  // the padding's diagonal block is still to come
+  const size_t base = out_starts ? out_starts[b] : 0;
   uint32_t count = 0;
-  const size_t first = out_starts ? out_starts[b] : 0;
-  for (;;) {
-    uint32_t c = own ? b : 0xffffffffu;
-    for (int p = 0; p < 3; ++p)
-      if (at[p] < end[p]) c = min(c, cols[at[p]] / 3);
-    if (c == 0xffffffffu) break;
-    if (c == b) own = false;
-    double* v = vals + (first + count) * 9;
-    for (int p = 0; p < 3; ++p)
-      for (; at[p] < end[p] && cols[at[p]] / 3 == c; ++at[p])
-        if (out_starts) v[3 * p + cols[at[p]] % 3] = scalars[at[p]];
-    if (out_starts) {
-      out[first + count] = c;
-      if (c == b)
-        for (int p = 0; p < 3; ++p)
-          if (3 * (uint64_t)b + p >= n) v[4 * p] = 1.0;
+  while (own || at[0] < end[0] || at[1] < end[1] || at[2] < end[2]) {
+    uint32_t col[3], block[3], limit = kNone;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      col[p] = at[p] + lane < end[p] ? cols[at[p] + lane] : kNone;
+      block[p] = col[p] == kNone ? kNone : col[p] / 3;
+      const uint32_t last = __shfl_sync(0xffffffffu, block[p], 31);
+      if (at[p] + 32 < end[p]) limit = min(limit, last);
     }
-    ++count;
+    unsigned lead[3];
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const uint32_t before = __shfl_up_sync(0xffffffffu, block[p], 1);
+      bool first = block[p] < limit && (lane == 0 || before != block[p]);
+#pragma unroll
+      for (int q = 0; q < p; ++q) {
+        const uint32_t k = lanes_below(block[q], block[p]);
+        if (__shfl_sync(0xffffffffu, block[q], k & 31) == block[p] && k < 32) first = false;
+      }
+      lead[p] = __ballot_sync(0xffffffffu, first);
+    }
+    const bool own_now = own && b < limit;
+    const bool own_lead =
+        own_now && !__any_sync(0xffffffffu, block[0] == b || block[1] == b || block[2] == b);
+    // the place of block `key` (every lane asks together)
+    auto place = [&](uint32_t key) {
+      uint32_t k = count + (own_lead && b < key);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        const uint32_t below = lanes_below(block[q], key);
+        k += __popc(below < 32 ? lead[q] & ((1u << below) - 1u) : lead[q]);
+      }
+      return k;
+    };
+    if (out_starts) {
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const size_t k = base + place(block[p]);
+        if (block[p] < limit) {
+          if (lead[p] >> lane & 1u) out[k] = block[p];
+          vals[k * 9 + 3 * p + col[p] % 3] = scalars[at[p] + lane];
+        }
+      }
+      if (own_now) {
+        const size_t k = base + place(b);
+        if (lane == 0) {
+          if (own_lead) out[k] = b;
+          for (int p = 0; p < 3; ++p)
+            if (3 * (uint64_t)b + p >= n) vals[k * 9 + 4 * p] = 1.0;
+        }
+      }
+    }
+    count += __popc(lead[0]) + __popc(lead[1]) + __popc(lead[2]) + own_lead;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) at[p] += __popc(__ballot_sync(0xffffffffu, block[p] < limit));
+    if (own_now) own = false;
   }
-  if (!out_starts) out[b] = count;
+  if (!out_starts && lane == 0) out[b] = count;
 }
 
 // Copies listed blocks out of (gather) or back into (scatter) a block array.
@@ -1037,7 +1092,7 @@ __global__ void set_values_kernel(size_t count, const uint32_t* __restrict__ idx
 sf_status setup_padded_blocks(cudaStream_t st, uint64_t n, uint32_t rows, const uint64_t* rs, const uint32_t* cols,
                               const double* scalars, const uint32_t* out_starts, uint32_t* out, double* vals) {
   if (rows == 0) return SF_OK;
-  padded_blocks_kernel<<<(rows + 127) / 128, 128, 0, st>>>(n, rows, rs, cols, scalars, out_starts, out, vals);
+  padded_blocks_kernel<<<(rows + 3) / 4, 128, 0, st>>>(n, rows, rs, cols, scalars, out_starts, out, vals);
   return cuda_check(cudaGetLastError(), "padded blocks");
 }
 
