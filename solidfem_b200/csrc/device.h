@@ -28,6 +28,7 @@ struct DevBsr {
   uint32_t group_blocks = 0;   // the largest group's block count
   uint32_t group_rows = 0;     // the largest group's row count
   int lanes_per_row = 32;      // lanes sharing one row: 32, 16, 8 or 4
+  uint32_t longest_row = 0;    // blocks of the longest row
   // SELL-32 copy for operators with many rows: slices of 32 rows (rows sorted by block count
   // inside windows of kSellWindow rows), one thread per row. Each lane reads its row in chunks of
   // U = sell_chunk_blocks(rb * cb, value bytes) consecutive blocks, 144 bytes of values stored as
@@ -86,6 +87,19 @@ bool wants_split(const DevBsr& m, bool uniform_lanes);
 // more rows to a group than a warp multiplies at once.
 sf_status make_row_groups(struct DeviceSolver& s, DevBsr& m, const uint32_t* host_starts, size_t value_bytes,
                           bool one_pass = false);
+
+// Lanes to a row of the conjugate gradient's row-group product (and its check). Rows of 4 lanes, under
+// about 7 blocks on average (raw sparse systems), take teams of 8: a row of up to eight blocks is
+// summed in the order of 32 lanes, whose other lanes add zeros, with four rows to a warp instead of
+// one (45^3 cells under Jacobi: 39 -> 33 us an iteration). Where some row is long, 32 lanes finish it
+// in a quarter of the rounds, which shows only while few rows run beside it: 1,000 block rows, one of
+// 998 blocks, 24 us an iteration with 32 lanes and 33 with 8; 6,667 with one of 788, 37 and 41; of 260
+// blocks, 30 and 32; 30,375 with one of 1,000, 141 and 96.
+static const uint32_t kLongRow = 256, kFewRows = 8192;
+inline int product_lanes(const DevBsr& m) {
+  if (m.lanes_per_row != 4) return m.lanes_per_row;
+  return m.longest_row > kLongRow && m.rows <= kFewRows ? 32 : 8;
+}
 
 // The solver's scalar state, resident on the device so the iteration loop runs without host
 // round trips; kernels read `status` and exit early once the solve has ended.

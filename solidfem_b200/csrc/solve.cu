@@ -170,6 +170,8 @@ sf_status make_row_groups(DeviceSolver& s, DevBsr& m, const uint32_t* starts, si
   m.group_bytes = max_bytes;
   m.group_blocks = max_blocks;
   m.group_rows = max_rows;
+  m.longest_row = 0;
+  for (uint32_t i = 0; i < m.rows; ++i) m.longest_row = std::max(m.longest_row, starts[i + 1] - starts[i]);
   if (sf_status e = dev_alloc(s, (void**)&m.groups, std::max<size_t>(1, g.size()) * sizeof(uint4))) return e;
   if (!g.empty()) copy_h2d(s, m.groups, g.data(), g.size() * sizeof(uint4));
   return cuda_check(cudaStreamSynchronize(s.stream), "row groups");
@@ -475,11 +477,7 @@ sf_status solver_enqueue_iteration(DeviceSolver& s) {
     launch_body<sell_pcg_spmv_dot_kernel>(grid, kThreads, 0, st, A, s.p, s.ap, s.partials, s.state);
     launch_body<pcg_update_kernel>(grid_for_reduction(s.n), kReduceThreads, 0, st, s.n, s.p, s.ap, s.x, s.r, s.partials, s.state);
     launch_body<sell_pcg_check_kernel>(grid, kThreads, 0, st, A, s.x, s.rhs, s.r, s.partials, s.state);
-  } else switch (s.system.lanes_per_row) {
-    // Short rows (under about 7 blocks, raw sparse systems) take teams of eight as well: a row of up
-    // to eight blocks is summed in the order of 32 lanes, whose other lanes add zeros, with four rows
-    // to a warp instead of one (45^3 cells under Jacobi: 39 -> 33 us an iteration).
-    case 4:
+  } else switch (product_lanes(s.system)) {
     case 8: launch_pcg_spmv_lpr<8>(s); break;
     case 16: launch_pcg_spmv_lpr<16>(s); break;
     default: launch_pcg_spmv_lpr<32>(s); break;

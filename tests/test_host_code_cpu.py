@@ -11,17 +11,20 @@ NATIVE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "native")
 
 
 def program(folder, name):
-    """tests/native/<name>.cpp with the library's <name>.cpp."""
+    """tests/native/<name>.cpp, with the library's <name>.cpp where there is one."""
     out = str(folder / name)
+    library = os.path.join(b.CSRC, name + ".cpp")
     subprocess.run([b.CXX, "-std=c++17", "-O1", "-fopenmp", "-Wno-unused-function", "-I" + NATIVE, "-I" + b.CSRC,
                     "-I" + os.path.join(b.CUDA, "include"), os.path.join(NATIVE, name + ".cpp"),
-                    os.path.join(b.CSRC, name + ".cpp"), "-o", out], check=True, capture_output=True, text=True)
+                    *([library] if os.path.exists(library) else []), "-o", out],
+                   check=True, capture_output=True, text=True)
     return out
 
 
 def run(*command):
     r = subprocess.run([str(c) for c in command], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
 
 
 @pytest.fixture(scope="module")
@@ -56,3 +59,15 @@ def test_the_longer_graph_is_made_where_it_pays(iterations, case):
     to go and does not make it, solves of 100 and 211 do. 14 kernels: worth 224, the sixth solve of 39
     has seen 195, the seventh more."""
     run(iterations, case)
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    return program(tmp_path_factory.mktemp("rules"), "rules")
+
+
+@pytest.mark.parametrize("lanes,rows,longest,expected", [
+    (4, 30375, 7, 8), (4, 1000, 256, 8), (4, 1000, 257, 32), (4, 8192, 1000, 32), (4, 8193, 1000, 8),
+    (8, 1000, 1000, 8), (16, 1000, 7, 16), (32, 30375, 7, 32)])
+def test_lanes_of_short_rows_and_of_a_few_long_ones(rules, lanes, rows, longest, expected):
+    assert int(run(rules, "product_lanes", lanes, rows, longest)) == expected
