@@ -643,7 +643,7 @@ __global__ void patch_fit_kernel(const double* __restrict__ nodes, uint32_t firs
   double scale = 0.0;
   bool any = false;
   for (uint32_t k = o0; k < o1; ++k) {
-    size_t base = (size_t)incident[k] * points;
+    size_t base = (size_t)(incident[k] >> 4) * points;
     for (int q = 0; q < points; ++q) {
       size_t pq = base + q;
       double E = pmat[pq * 2], nu = pmat[pq * 2 + 1];
@@ -664,7 +664,7 @@ __global__ void patch_fit_kernel(const double* __restrict__ nodes, uint32_t firs
   for (int i = 0; i < 4; ++i)
     for (int k = 0; k < 6; ++k) rhs[i][k] = 0.0;
   for (uint32_t k = o0; k < o1; ++k) {
-    size_t base = (size_t)incident[k] * points;
+    size_t base = (size_t)(incident[k] >> 4) * points;
     for (int q = 0; q < points; ++q) {
       size_t pq = base + q;
       double t[4] = {1.0, (ppos[pq * 3] - c[0]) / scale, (ppos[pq * 3 + 1] - c[1]) / scale, (ppos[pq * 3 + 2] - c[2]) / scale};
@@ -741,26 +741,27 @@ __global__ void nodal_field_kernel(const double* __restrict__ nodes, const uint3
   vm[n] = sqrt(0.5 * (a0 * a0 + b0 * b0 + c0 * c0) + 3.0 * (s[3] * s[3] + s[4] * s[4] + s[5] * s[5]));
 }
 
-// disp (zeros) at every free row's node from the free-DOF solution.
-__global__ void scatter_displacements_kernel(const double* __restrict__ x, const uint32_t* __restrict__ row_node,
+__global__ void scatter_displacements_kernel(const double* __restrict__ x, const uint32_t* __restrict__ free,
                                              size_t count, double* __restrict__ disp) {
   const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < count) disp[(size_t)row_node[i / 3] * 3 + i % 3] = x[i];
+  if (i >= count) return;
+  const uint32_t f = free[i / 3];
+  disp[i] = f == 0xffffffffu ? 0.0 : x[(size_t)f * 3 + i % 3];
 }
 
-// The recovery's incidence (results.rs:414-435) from the assembly's: each node's (element, local
-// node) in element order, and each midside node's first element and edge slot. A vertex's elements
-// are its node's elements as they stand (a vertex is only ever a corner).
+// The recovery's incidence (results.rs:414-435): each node's (element, local node) in element order,
+// over its elements, and each midside node's first element and edge slot. A vertex is only ever a
+// corner, so its node's list is the vertex's too.
 __global__ void node_incidence_kernel(const uint32_t* __restrict__ tets, uint32_t nodes, uint32_t vertices,
-                                      const uint32_t* __restrict__ inc_start, const uint32_t* __restrict__ inc,
-                                      uint32_t* __restrict__ node_incident, uint32_t* __restrict__ midside_first) {
+                                      const uint32_t* __restrict__ inc_start, uint32_t* __restrict__ incident,
+                                      uint32_t* __restrict__ midside_first) {
   const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nodes) return;
   for (uint32_t k = inc_start[n]; k < inc_start[n + 1]; ++k) {
-    const uint32_t e = inc[k];
+    const uint32_t e = incident[k];
     uint32_t a = 0;
     while (a < 9 && tets[(size_t)e * 10 + a] != n) ++a;
-    node_incident[k] = (e << 4) | a;
+    incident[k] = (e << 4) | a;
     if (n >= vertices && k == inc_start[n]) midside_first[n - vertices] = (e << 3) | (a - 4);
   }
 }
@@ -785,17 +786,18 @@ __global__ void pack_points_kernel(const double* __restrict__ stress, const doub
 
 }  // namespace
 
-sf_status launch_scatter_displacements(const double* x, const uint32_t* row_node, size_t rows, double* disp,
+sf_status launch_scatter_displacements(const double* x, const uint32_t* free, size_t node_count, double* disp,
                                        cudaStream_t stream) {
-  if (rows == 0) return SF_OK;
-  scatter_displacements_kernel<<<(unsigned)((3 * rows + 255) / 256), 256, 0, stream>>>(x, row_node, 3 * rows, disp);
+  if (node_count == 0) return SF_OK;
+  scatter_displacements_kernel<<<(unsigned)((3 * node_count + 255) / 256), 256, 0, stream>>>(x, free, 3 * node_count,
+                                                                                             disp);
   return cuda_check(cudaGetLastError(), "scatter displacements");
 }
 
-sf_status launch_node_incidence(const AssemblyDevice& a, uint32_t node_count, uint32_t vertex_count, uint32_t* incident,
-                                uint32_t* midside_first, cudaStream_t stream) {
-  node_incidence_kernel<<<(node_count + 127) / 128, 128, 0, stream>>>(a.tets, node_count, vertex_count, a.inc_start,
-                                                                      a.inc, incident, midside_first);
+sf_status launch_node_incidence(const AssemblyDevice& a, RecoveryDevice& r, uint32_t node_count, uint32_t vertex_count,
+                                cudaStream_t stream) {
+  node_incidence_kernel<<<(node_count + 127) / 128, 128, 0, stream>>>(a.tets, node_count, vertex_count, r.node_offsets,
+                                                                      r.node_incident, r.midside_first);
   return cuda_check(cudaGetLastError(), "recovery incidence");
 }
 
@@ -823,8 +825,8 @@ sf_status launch_recovery_elements(const AssemblyDevice& a, const MaterialSpec& 
 sf_status launch_recovery_fits(const AssemblyDevice& a, RecoveryDevice& r, uint32_t first, uint32_t end,
                                cudaStream_t stream) {
   if (end <= first) return SF_OK;
-  patch_fit_kernel<<<(end - first + 127) / 128, 128, 0, stream>>>(a.nodes, first, end, a.points, r.vertex_offsets,
-                                                                  r.vertex_incident, r.point_stress, r.point_pos,
+  patch_fit_kernel<<<(end - first + 127) / 128, 128, 0, stream>>>(a.nodes, first, end, a.points, r.node_offsets,
+                                                                  r.node_incident, r.point_stress, r.point_pos,
                                                                   r.point_mat, r.fits, r.has_fit);
   return cuda_check(cudaGetLastError(), "recovery patch fits");
 }

@@ -141,7 +141,7 @@ struct DevLevel {
   double theta = 0;
   std::vector<std::pair<double, double>> steps;
   // vectors of the vector precision
-  void *b = nullptr, *x = nullptr, *res = nullptr, *z = nullptr, *d0 = nullptr, *d1 = nullptr,
+  void *b = nullptr, *x = nullptr, *res = nullptr, *d0 = nullptr, *d1 = nullptr,
        *post_x = nullptr, *tmp = nullptr;
 };
 
@@ -351,9 +351,8 @@ struct RecoveryDevice {
   double* point_pos = nullptr;    // tet_count x points x 3
   double* point_mat = nullptr;    // tet_count x points x 2
   double* node_candidate = nullptr;  // tet_count x 10 x 7: stress and von Mises at each node
-  const uint32_t* vertex_offsets = nullptr;  // vertex_count + 1 (the assembly's incidence)
-  const uint32_t* vertex_incident = nullptr; // elements touching each vertex, ascending
-  const uint32_t* node_offsets = nullptr;    // node_count + 1: (element, local node) incidence
+  uint32_t* free = nullptr;            // node_count: free index or FIXED
+  uint32_t* node_offsets = nullptr;    // node_count + 1: (element, local node) incidence
   uint32_t* node_incident = nullptr;   // (element << 4) | local node, ascending element
   double* fits = nullptr;         // vertex_count x 28: centre (3), scale, coefficients (4 x 6)
   int* has_fit = nullptr;         // vertex_count
@@ -373,13 +372,17 @@ sf_status launch_recovery_fits(const AssemblyDevice& a, RecoveryDevice& r, uint3
                                cudaStream_t stream);
 sf_status launch_recovery_field(const AssemblyDevice& a, RecoveryDevice& r, uint32_t node_count,
                                 uint32_t vertex_count, cudaStream_t stream);
-// The displacement of every free row's node from the free-DOF solution, into zeros.
-sf_status launch_scatter_displacements(const double* x, const uint32_t* row_node, size_t rows, double* disp,
+// The displacement of every mesh node from the free-DOF solution (zero at fixed nodes).
+sf_status launch_scatter_displacements(const double* x, const uint32_t* free, size_t node_count, double* disp,
                                        cudaStream_t stream);
-// The recovery's per-node (element << 4 | local node) list, laid out as a.inc, and its midsides'
-// first elements, from the assembly's incidence.
-sf_status launch_node_incidence(const AssemblyDevice& a, uint32_t node_count, uint32_t vertex_count, uint32_t* incident,
-                                uint32_t* midside_first, cudaStream_t stream);
+// Each node's elements, ascending: start (nodes + 1) and inc (10 x tets); enqueued on `stream`
+// (mesh_device.cu).
+sf_status device_incidence(cudaStream_t stream, const uint32_t* tets10, size_t tets, size_t nodes, uint32_t* start,
+                           uint32_t* inc);
+// r.node_incident from each node's elements to (element << 4) | local node, in place, and the
+// midsides' first elements.
+sf_status launch_node_incidence(const AssemblyDevice& a, RecoveryDevice& r, uint32_t node_count, uint32_t vertex_count,
+                                cudaStream_t stream);
 // Points [first, first + count) as sf_point_stress records.
 sf_status launch_pack_points(const RecoveryDevice& r, int points, size_t first, size_t count, void* out,
                              cudaStream_t stream);

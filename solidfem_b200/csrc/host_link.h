@@ -83,16 +83,18 @@ sf_status copy_out(const DeviceSolver& d, void* dst, size_t bytes, size_t chunk,
   return e ? e : end;
 }
 
-// Host bytes to device memory and to `keep`, ordinary memory of the study's; `src` may be reused on return.
+// Host bytes to device memory and to `keep`, ordinary memory of the study's (null where `src` is that
+// already); `src` may be reused on return.
 inline sf_status copy_in(const DeviceSolver& d, void* dst, const void* src, void* keep, size_t bytes, int threads) {
   if (bytes < kSmallCopy) {
-    std::memcpy(keep, src, bytes);
-    if (bytes) copy_h2d(d, dst, keep, bytes);  // not from src: a page-locked one is read when the stream gets there
+    if (keep) std::memcpy(keep, src, bytes);
+    // not from a caller's src: a page-locked one is read when the stream gets there
+    if (bytes) copy_h2d(d, dst, keep ? keep : src, bytes);
     return SF_OK;
   }
   Staging st(std::min(kCopyChunk, bytes));
   if (!st.ok) {
-    std::memcpy(keep, src, bytes);
+    if (keep) std::memcpy(keep, src, bytes);
     copy_h2d(d, dst, src, bytes);
     return cuda_check(cudaStreamSynchronize(d.stream), "copy to the device");
   }
@@ -103,7 +105,7 @@ inline sf_status copy_in(const DeviceSolver& d, void* dst, const void* src, void
     host_copy(st.buf[i & 1], (const char*)src + at, len, threads);
     copy_h2d(d, (char*)dst + at, st.buf[i & 1], len);
     cudaEventRecord(st.done[i & 1], d.stream);
-    host_copy((char*)keep + at, (const char*)src + at, len, threads);
+    if (keep) host_copy((char*)keep + at, (const char*)src + at, len, threads);
   }
   const sf_status end = cuda_check(cudaStreamSynchronize(d.stream), "copy to the device");
   return e ? e : end;

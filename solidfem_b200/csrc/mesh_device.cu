@@ -518,20 +518,22 @@ __global__ void face_emit_kernel(const uint32_t* __restrict__ off, const unsigne
 }
 
 // ------------------------------------------------------------------ host orchestration
-// Device buffers of one build on its own non-blocking stream, from the device's stream-ordered
-// pool; everything not handed to the mesh is freed on the stream when the build ends.
+// Device buffers of one build on its own non-blocking stream (or, `borrowed`, on one that goes on),
+// from the device's stream-ordered pool; everything not handed to the mesh is freed on the stream
+// when the build ends.
 struct Build {
   int device = 0, prev = 0;
   cudaStream_t stream = nullptr;
+  bool borrowed = false;
   std::vector<void*> temps;
   cudaError_t err = cudaSuccess;
   ~Build() {
     for (void* p : temps) cudaFreeAsync(p, stream);
-    if (stream) {
+    if (stream && !borrowed) {
       cudaStreamSynchronize(stream);
       cudaStreamDestroy(stream);
     }
-    cudaSetDevice(prev);
+    if (!borrowed) cudaSetDevice(prev);
   }
   template <typename T>
   T* alloc(size_t count, bool keep = false) {
@@ -936,7 +938,31 @@ __global__ void __launch_bounds__(32 * kPatternWarps) pattern_rows_kernel(
   }
 }
 
+// Each node's elements, ascending, of tets10's `nt` entries: start (nodes + 1) and inc (nt).
+sf_status enqueue_incidence(Build& b, const uint32_t* tets10, size_t nt, size_t nodes, uint32_t* start, uint32_t* inc) {
+  uint32_t* count = b.alloc<uint32_t>(nodes);
+  uint32_t* cursor = b.alloc<uint32_t>(nodes);
+  if (b.err) return scan_failed(b);
+  cudaMemsetAsync(count, 0, nodes * 4, b.stream);
+  incidence_count_kernel<<<grid_of(nt), kT, 0, b.stream>>>(tets10, nt, count);
+  if (!scan(b, count, start, nodes)) return scan_failed(b);
+  cudaMemcpyAsync(cursor, start, nodes * 4, cudaMemcpyDeviceToDevice, b.stream);
+  incidence_fill_kernel<<<grid_of(nt), kT, 0, b.stream>>>(tets10, nt, cursor, inc);
+  incidence_sort_kernel<<<grid_of(nodes), kT, 0, b.stream>>>(start, inc, nodes);
+  return SF_OK;
+}
+
 }  // namespace
+
+sf_status device_incidence(cudaStream_t stream, const uint32_t* tets10, size_t tets, size_t nodes, uint32_t* start,
+                           uint32_t* inc) {
+  Build b;
+  b.stream = stream;
+  b.borrowed = true;
+  if (sf_status e = enqueue_incidence(b, tets10, 10 * tets, nodes, start, inc)) return e;
+  if (cudaError_t e = cudaGetLastError()) return cuda_fail(e, "incidence");
+  return SF_OK;
+}
 
 sf_status device_pattern(const Mesh& mesh, const vector<uint32_t>& free, size_t free_count, DevicePattern& out,
                          vector<uint32_t>& host_starts, bool* fallback) {
@@ -959,8 +985,6 @@ sf_status device_pattern(const Mesh& mesh, const vector<uint32_t>& free, size_t 
   keep(&out.cursor, free_count);
   keep(&out.starts, free_count + 1);
   uint32_t* dfree = b.alloc<uint32_t>(nn);
-  uint32_t* count = b.alloc<uint32_t>(nn);
-  uint32_t* cursor = b.alloc<uint32_t>(nn);
   uint32_t* rows = b.alloc<uint32_t>(free_count);
   unsigned* overflow = b.alloc<unsigned>(1);
   if (b.err) {
@@ -969,17 +993,11 @@ sf_status device_pattern(const Mesh& mesh, const vector<uint32_t>& free, size_t 
   }
   cudaStream_t st = b.stream;
   cudaMemcpyAsync(dfree, free.data(), nn * 4, cudaMemcpyHostToDevice, st);
-  cudaMemsetAsync(count, 0, nn * 4, st);
   cudaMemsetAsync(overflow, 0, 4, st);
-  incidence_count_kernel<<<grid_of(nt), kT, 0, st>>>(mesh.dev->tets, nt, count);
-  if (!scan(b, count, out.inc_start, nn)) {
-    const sf_status e = scan_failed(b);
+  if (sf_status e = enqueue_incidence(b, mesh.dev->tets, nt, nn, out.inc_start, out.inc)) {
     release();
     return e;
   }
-  cudaMemcpyAsync(cursor, out.inc_start, nn * 4, cudaMemcpyDeviceToDevice, st);
-  incidence_fill_kernel<<<grid_of(nt), kT, 0, st>>>(mesh.dev->tets, nt, cursor, out.inc);
-  incidence_sort_kernel<<<grid_of(nn), kT, 0, st>>>(out.inc_start, out.inc, nn);
   row_node_kernel<<<grid_of(nn), kT, 0, st>>>(dfree, out.inc_start, nn, out.row_node, out.cursor);
   const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((free_count + kPatternWarps - 1) / kPatternWarps,
                                                                        148 * 16));

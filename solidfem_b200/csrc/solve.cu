@@ -401,7 +401,7 @@ sf_status solver_upload_hierarchy(DeviceSolver& s, const std::vector<HostLevel>&
       L.steps.push_back({next * rho, 2.0 * next / delta});
       rho = next;
     }
-    void** vecs[] = {&L.b, &L.x, &L.res, &L.z, &L.d0, &L.d1, &L.post_x, &L.tmp};
+    void** vecs[] = {&L.b, &L.x, &L.res, &L.d0, &L.d1, &L.post_x, &L.tmp};
     for (void** v : vecs)
       if (sf_status e = dev_alloc(s, v, (size_t)L.n * V)) return e;
   }

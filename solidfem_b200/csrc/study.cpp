@@ -1117,12 +1117,12 @@ static sf_status builder_assemble(sf_builder* b, uint64_t max_elements, sf_cance
         return me;
       }
     }
-    // The element stiffness buffer and the rows' cursors have served; free them for the solve. The
-    // incidence and the rows' nodes stay for the recovery and the displacements.
-    dev_free(s, a.ke);
-    dev_free(s, a.cursor);
+    // The element stiffness buffer and the assembly map have served; free them for the solve (a
+    // recovery makes the incidence again: kept, it would count against the study's memory budget).
+    for (void* p : {(void*)a.ke, (void*)a.inc_start, (void*)a.inc, (void*)a.row_node, (void*)a.cursor})
+      dev_free(s, p);
     a.ke = nullptr;
-    a.cursor = nullptr;
+    a.inc_start = a.inc = a.row_node = a.cursor = nullptr;
   }
   return SF_OK;
 }
@@ -1536,15 +1536,16 @@ sf_status sf_study_displacements(const sf_study* s, double* out) {
   const size_t nn = s->free.size();
   // Large fields are spread over the nodes on the device and come to the caller's memory through
   // pinned buffers; small ones, or when the device has no room for one, are spread here.
-  double* field = nullptr;
+  double* field = nullptr;  // and the nodes' free numbers behind it
   pool_setup(d.device);
-  if (nn >= kDeviceFieldNodes && cudaMallocAsync((void**)&field, nn * 24, d.stream) != cudaSuccess) {
+  if (nn >= kDeviceFieldNodes && cudaMallocAsync((void**)&field, nn * 28, d.stream) != cudaSuccess) {
     cudaGetLastError();
     field = nullptr;
   }
   if (field) {
-    cudaMemsetAsync(field, 0, nn * 24, d.stream);
-    sf_status e = launch_scatter_displacements(d.x, s->asmdev.row_node, s->free_count, field, d.stream);
+    uint32_t* numbers = (uint32_t*)(field + 3 * nn);
+    sf_status e = copy_in(d, numbers, s->free.data(), nullptr, nn * 4, host_threads(s));
+    if (!e) e = launch_scatter_displacements(d.x, numbers, nn, field, d.stream);
     if (!e) e = copy_out(d, out, nn * 24, kCopyChunk, host_threads(s), [&](size_t at, size_t) { return (char*)field + at; });
     cudaFreeAsync(field, d.stream);
     if (e) return e;
@@ -1567,8 +1568,8 @@ sf_status sf_study_report(const sf_study* s, sf_report* out) {
 }
 
 // Device stress recovery (Recovery, results.rs:97-124, 376-539). The incidence lists every
-// recovery of a study reads are made once, from the assembly's; a recovery snapshots the displacements on
-// the device and advances in the reference's units of work (each element, then each vertex's
+// recovery of a study reads are made once, on the device; a recovery snapshots the displacements
+// there and advances in the reference's units of work (each element, then each vertex's
 // patch fit); the nodal field is made when both are done.
 static sf_status recovery_tables(sf_study* s) {
   RecoveryDevice& r = s->rec;
@@ -1576,13 +1577,18 @@ static sf_status recovery_tables(sf_study* s) {
   DeviceSolver& d = s->solver;
   const Mesh& m = s->model.mesh;
   const size_t nn = m.nodes.size(), nv = m.vertex_count;
-  sf_status e = dev_alloc(d, (void**)&r.node_incident, std::max<size_t>(1, 10 * m.tets.size()) * 4);
+  sf_status e = dev_alloc(d, (void**)&r.free, nn * 4);
+  if (!e) e = dev_alloc(d, (void**)&r.node_offsets, (nn + 1) * 4);
+  if (!e) e = dev_alloc(d, (void**)&r.node_incident, std::max<size_t>(1, 10 * m.tets.size()) * 4);
   if (!e) e = dev_alloc(d, (void**)&r.midside_first, std::max<size_t>(1, nn - nv) * 4);
-  if (e) return e;
-  r.vertex_offsets = r.node_offsets = s->asmdev.inc_start;
-  r.vertex_incident = s->asmdev.inc;
-  if ((e = launch_node_incidence(s->asmdev, (uint32_t)nn, (uint32_t)nv, r.node_incident, r.midside_first, d.stream)))
+  if (!e) e = copy_in(d, r.free, s->free.data(), nullptr, nn * 4, host_threads(s));
+  if (!e) e = device_incidence(d.stream, s->asmdev.tets, m.tets.size(), nn, r.node_offsets, r.node_incident);
+  if (!e) e = launch_node_incidence(s->asmdev, r, (uint32_t)nn, (uint32_t)nv, d.stream);
+  if (e) {
+    for (void* p : {(void*)r.free, (void*)r.node_offsets, (void*)r.node_incident, (void*)r.midside_first}) dev_free(d, p);
+    r = RecoveryDevice();
     return e;
+  }
   d.launches += 1;
   r.ready = true;
   return SF_OK;
@@ -1629,7 +1635,7 @@ static sf_status recovery_begin(sf_study* s, sf_recovery** out) {
   if (!e) e = alloc((void**)&r.has_fit, nv * 4);
   if (!e) e = alloc((void**)&r.nodal_stress, nn * 48);
   if (!e) e = alloc((void**)&r.nodal_vm, nn * 8);
-  if (!e) e = launch_scatter_displacements(d.x, s->asmdev.row_node, s->free_count, r.disp, d.stream);
+  if (!e) e = launch_scatter_displacements(d.x, r.free, nn, r.disp, d.stream);
   if (!e && !s->model.prescribed.empty()) {
     // the prescribed components, exact
     vector<uint32_t> idx;
