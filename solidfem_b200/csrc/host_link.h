@@ -53,7 +53,7 @@ struct Staging {
 // bytes [at, at + len) of a chunk, enqueueing what makes them on d.stream first.
 template <class F>
 sf_status copy_out(const DeviceSolver& d, void* dst, size_t bytes, size_t chunk, int threads, F&& from) {
-  if (bytes < kSmallCopy) {
+  if (bytes < kSmallCopy && bytes <= chunk) {
     if (bytes) copy_d2h(d, dst, from(0, bytes), bytes);
     return cuda_check(cudaStreamSynchronize(d.stream), "copy to the host");
   }

@@ -34,6 +34,21 @@ void round_trip(size_t n, int pinned) {
   CHECK(cudaGetLastError() == cudaSuccess);  // a refused allocation is nobody else's error
 }
 
+// A small array put together in less than its size at a time.
+void small_chunks(size_t n) {
+  DeviceSolver d;
+  std::vector<char> src = pattern(n), half[2], out(n);
+  for (auto& h : half) h.resize(176);
+  int turn = 0;
+  CHECK(copy_out(d, out.data(), n, 176, 3, [&](size_t at, size_t len) {
+          CHECK(len <= 176);
+          char* to = half[turn ^= 1].data();
+          fake::stream.push_back([=, &src] { std::memcpy(to, src.data() + at, len); });
+          return to;
+        }) == SF_OK);
+  CHECK(out == src);
+}
+
 // The caller's array may be reused once copy_in has returned, page-locked or not.
 void reuse(size_t n) {
   DeviceSolver d;
@@ -57,5 +72,6 @@ int main(int argc, char** argv) {
   if (what == "no-pinned") round_trip(n, 0);
   if (what == "one-pinned") round_trip(n, 1);
   if (what == "reuse") reuse(n);
+  if (what == "small-chunks") small_chunks(n);
   return 0;
 }

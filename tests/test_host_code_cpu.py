@@ -43,6 +43,11 @@ def test_a_load_vector_may_be_reused_once_it_was_taken(host_link, size):
     run(host_link, "reuse", size)
 
 
+@pytest.mark.parametrize("size", [88, 176, 264, 2112])
+def test_a_small_array_may_cross_in_smaller_chunks(host_link, size):
+    run(host_link, "small-chunks", size)
+
+
 @pytest.fixture(scope="module")
 def iterations(tmp_path_factory):
     return program(tmp_path_factory.mktemp("iterations"), "iterations")
