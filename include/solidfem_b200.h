@@ -437,6 +437,7 @@ sf_status sf_study_system_multiply(sf_study* study, const double* x, double* y);
  * allocates two device buffers per call and copies through the host.) The reduction's scratch is
  * a static 262,400-byte device array in this library, one per device.
  *
+ * - A vector's product and energy have the same bits whatever count, and whatever its place.
  * - count at most 8; a larger count is refused with SF_INVALID_ARGUMENT before any work. count 0
  *   does nothing. x, y and energy: 8-byte-aligned device (or managed) memory of the study's
  *   device, not overlapping; x and y hold count * free_dofs doubles, energy count doubles, each

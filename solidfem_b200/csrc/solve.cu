@@ -733,6 +733,7 @@ sf_status solver_read_state(DeviceSolver& s, PcgState* out) {
 // (different streams, different studies, different host threads) race on it.
 constexpr int kEnergyMaxVectors = 8;
 constexpr int kEnergyMaxBlocks = 4096;  // blocks per vector of one launch
+constexpr int kEnergyOneBlocks = 1024;  // of a launch for one vector, whose sums the others repeat
 constexpr size_t kEnergyTicketBytes = 256;
 constexpr size_t kEnergyScratchBytes = kEnergyTicketBytes + (size_t)kEnergyMaxVectors * kEnergyMaxBlocks * sizeof(double);
 constexpr int kEnergyMaxDevices = 64;
@@ -768,15 +769,17 @@ __global__ void __launch_bounds__(kThreads) sell_energy_one_kernel(SellOp<double
 // sell_kernel sums it, so the operator's stream (76 bytes a block) is read from memory once for
 // all the vectors. A block is W slices by G groups of K vectors, a warp each: the G warps of a
 // slice read its stream from L1. The x gathers bound it (3 K loads a block of about 25 sectors,
-// L2 latency), so more than four vectors run as two groups of half the accumulators: 16 warps of
-// K = 4 hide more of it than 8 of K = 8. Gate plate (201,000 rows, 394 MB of operator), 8 vectors:
+// L2 latency), so more than four vectors run as two groups of half the accumulators: 12 resident warps
+// of K = 4 hide more of it than 8 of K = 8. Gate plate (201,000 rows, 394 MB of operator), 8 vectors:
 // 487 us a call with a grid row per vector (the operator read eight times), 340 us with K = 8 in
-// one thread, 224 us with two groups of four (the floor of its bytes is 72 us); 4 vectors 242 -> 125
-// us, 2 vectors 131 -> 97 us.
+// one thread, 208 us with two groups of four (the floor of its bytes is 72 us); 4 vectors 234 -> 116
+// us, 2 vectors 119 -> 86 us (one call after another).
 template <int K, int G, int W>
 __global__ void __launch_bounds__(32 * W * G) sell_energy_kernel(SellOp<double> A, const double* __restrict__ x,
                                                              double* __restrict__ y, uint32_t n, int count,
-                                                             double* __restrict__ energy, unsigned char* scratch) {
+                                                             uint32_t blocks, double* __restrict__ energy,
+                                                             unsigned char* scratch) {
+  constexpr int SHARES = kWarps / W;  // blocks to a virtual block
   constexpr int LEN = 9, U = sell_chunk_blocks(LEN, 8), VEC = 2, NV = U * LEN / VEC;
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int first = (int)(warp / W) * K;  // this warp's vectors: first .. first + K - 1, those below count
@@ -786,7 +789,8 @@ __global__ void __launch_bounds__(32 * W * G) sell_energy_kernel(SellOp<double> 
   double local[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) local[k] = 0.0;
-  for (uint32_t s = blockIdx.x * W + warp % W; s < A.nslices; s += gridDim.x * W) {
+  const uint32_t vb = blockIdx.x / SHARES, share = blockIdx.x % SHARES;
+  for (uint32_t s = vb * kWarps + share + SHARES * (warp % W); s < A.nslices; s += blocks * kWarps) {
     const uint32_t slot = s * 32 + lane;
     const uint32_t row = A.rows[slot], len = A.len[slot], base = A.start[s];
     double acc[K][3];
@@ -845,9 +849,11 @@ __global__ void __launch_bounds__(32 * W * G) sell_energy_kernel(SellOp<double> 
             local[k] += xg[k][i] * acc[k][p];
           }
   }
-  // The energies: each warp's sums by shuffles, the block's slices in order, one partial per
-  // block and vector (vector k's at k * kEnergyMaxBlocks); the last block of the call sums each
-  // vector's partials, a warp per vector, in a fixed order. One ticket (vector 0's) serves the call.
+  // The energies in the order of finish_partials over `blocks` blocks of kWarps warps: each warp's sum
+  // by shuffles; the sums of a block's warps (every SHARES-th one of its virtual block's) in pairs as
+  // block_sum pairs them, one partial per block and vector; the last block of the call then pairs the
+  // shares and sums each vector's blocks, a warp per vector in the place of its kThreads threads. So an
+  // energy does not depend on the number of vectors in the call. One ticket (vector 0's) serves the call.
   __shared__ double sh[K * G][W];
   __shared__ bool last;
 #pragma unroll
@@ -860,10 +866,13 @@ __global__ void __launch_bounds__(32 * W * G) sell_energy_kernel(SellOp<double> 
   __syncthreads();
   double* partials = reinterpret_cast<double*>(scratch + kEnergyTicketBytes);
   if ((int)threadIdx.x < count) {
-    double v = sh[threadIdx.x][0];
-#pragma unroll
-    for (int w = 1; w < W; ++w) v += sh[threadIdx.x][w];
-    __stcg(partials + (size_t)threadIdx.x * kEnergyMaxBlocks + blockIdx.x, v);
+    const double* v = sh[threadIdx.x];
+    double t;
+    if constexpr (W == 2)
+      t = v[0] + v[1];
+    else
+      t = (v[0] + v[2]) + (v[1] + v[3]);
+    __stcg(partials + (size_t)threadIdx.x * kEnergyMaxBlocks + blockIdx.x, t);
     __threadfence();
   }
   __syncthreads();
@@ -873,12 +882,28 @@ __global__ void __launch_bounds__(32 * W * G) sell_energy_kernel(SellOp<double> 
   if (!last) return;
   __threadfence();
   for (int k = (int)warp; k < count; k += W * G) {
-    double v = 0.0;
-#pragma unroll 8
-    for (unsigned i = lane; i < gridDim.x; i += 32) v += __ldcg(partials + (size_t)k * kEnergyMaxBlocks + i);
+    const double* part = partials + (size_t)k * kEnergyMaxBlocks;
+    double v[kWarps];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
-    if (lane == 0) energy[k] = v;
+    for (int w = 0; w < kWarps; ++w) v[w] = 0.0;
+    for (uint32_t b0 = lane; b0 < blocks; b0 += kThreads) {
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {  // past the last block: zeros, which change nothing
+        const uint32_t b = b0 + 32 * w;
+        double t[SHARES];
+#pragma unroll
+        for (int i = 0; i < SHARES; ++i) t[i] = b < blocks ? __ldcg(part + (size_t)b * SHARES + i) : 0.0;
+        if constexpr (SHARES == 4)
+          v[w] += (t[0] + t[2]) + (t[1] + t[3]);
+        else
+          v[w] += t[0] + t[1];
+      }
+    }
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[w] += __shfl_xor_sync(kFull, v[w], o);
+    if (lane == 0) energy[k] = ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
   }
   if (threadIdx.x == 0) *ticket = 0u;
 }
@@ -901,9 +926,10 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(Op<double> A, const do
 
 // Row-group system, several vectors: K of them in one walk (blockIdx.y picks the K), so a group's
 // staged values are read once for all of them and each x gather round is K times as wide; rows are
-// summed as bsr_kernel sums them. One staging slot a warp (a warp has one group or few), eight warps
-// a block. 26,010 rows, 8 vectors: 118 -> 83 us a call, 3 vectors 53 -> 44; 3,240 rows, 8 vectors:
-// 37 -> 28 (with a grid row per vector before).
+// summed as bsr_kernel sums them. One staging slot a warp (a warp has one group or few) on energy_kernel's
+// grid, whose warps, blocks and sums these are: an energy does not depend on the number of vectors.
+// 26,010 rows, 8 vectors: 109 -> 68 us a call, 3 vectors 45 -> 38; 3,240 rows, 8 vectors: 29 -> 21
+// (with a grid row per vector before; one call after another).
 template <int LPR, int K>
 __global__ void __launch_bounds__(kThreads) energy_groups_kernel(Op<double> A, const double* __restrict__ x,
                                                                   double* __restrict__ y, uint32_t n, int count,
@@ -1020,16 +1046,17 @@ sf_status energy_setup(int device, unsigned char** out) {
   return SF_OK;
 }
 
+unsigned energy_one_blocks(uint32_t nslices) { return (unsigned)std::min(grid_for_slices(nslices), kEnergyOneBlocks); }
+
 template <int K, int G>
 void launch_energy_sell(const SellOp<double>& A, const double* x, double* y, uint32_t n, int count, double* energy,
                         unsigned char* scratch, cudaStream_t st) {
-  // A block per W slices, so the SMs that finish early take the next ones; above the scratch's
-  // slots every block takes the same number of them.
+  // A block per W slices (of the blocks of sell_energy_one_kernel, whose sums are formed), so the SMs
+  // that finish early take the next ones.
   constexpr int W = G == 1 ? 4 : 2;  // 128 threads, three resident blocks at about 166 registers
-  const unsigned want = std::max(1u, (A.nslices + W - 1) / W);
-  const unsigned rounds = (want + kEnergyMaxBlocks - 1) / kEnergyMaxBlocks;
-  const unsigned grid = (want + rounds - 1) / rounds;
-  sell_energy_kernel<K, G, W><<<grid, 32 * W * G, 0, st>>>(A, x, y, n, count, energy, scratch);
+  static_assert(kWarps == 8 && kWarps / 2 * kEnergyOneBlocks <= kEnergyMaxBlocks, "a partial per block");
+  const unsigned blocks = energy_one_blocks(A.nslices);
+  sell_energy_kernel<K, G, W><<<blocks * (kWarps / W), 32 * W * G, 0, st>>>(A, x, y, n, count, blocks, energy, scratch);
 }
 
 template <int LPR>
@@ -1037,7 +1064,7 @@ void launch_energy_lpr(const DevBsr& m, const double* x, double* y, uint32_t n, 
                        unsigned char* scratch, cudaStream_t st) {
   Op<double> A = op_of<double>(m);
   Shape sh = shape_of(A, true);
-  dim3 grid((unsigned)std::min(sh.grid, 1024), (unsigned)count);
+  dim3 grid((unsigned)std::min(sh.grid, kEnergyOneBlocks), (unsigned)count);
   energy_kernel<LPR><<<grid, sh.threads, sh.smem, st>>>(A, x, y, n, energy, scratch);
 }
 
@@ -1045,11 +1072,9 @@ template <int LPR, int K>
 void launch_energy_groups(const DevBsr& m, const double* x, double* y, uint32_t n, double* energy, int count,
                           unsigned char* scratch, cudaStream_t st) {
   Op<double> A = op_of<double>(m);
-  const size_t slot = slot_bytes(A);
-  const int warps = (int)std::max<size_t>(1, std::min<size_t>(kWarps, kSmemPerBlockTarget / slot));
-  const unsigned want = (A.ngroups + warps - 1) / warps;
-  const dim3 grid(std::max(1u, std::min<unsigned>(want, 1024)), (unsigned)((count + K - 1) / K));
-  energy_groups_kernel<LPR, K><<<grid, 32 * warps, slot * warps, st>>>(A, x, y, n, count, energy, scratch);
+  const Shape sh = shape_of(A, true);  // the blocks of energy_kernel, whose sums are formed
+  const dim3 grid((unsigned)std::min(sh.grid, kEnergyOneBlocks), (unsigned)((count + K - 1) / K));
+  energy_groups_kernel<LPR, K><<<grid, sh.threads, sh.smem / 2, st>>>(A, x, y, n, count, energy, scratch);
 }
 
 // Two to four vectors in one walk, five to eight in two of three or four.
@@ -1081,7 +1106,7 @@ sf_status solver_energy_products(DeviceSolver& s, const double* x, double* y, do
   if (m.sell) {
     SellOp<double> A = sell_of<double>(m);
     const int k = (int)count;
-    if (k == 1) sell_energy_one_kernel<<<std::min(grid_for_slices(m.nslices), 1024), kThreads, 0, s.stream>>>(A, x, y, energy, scratch);
+    if (k == 1) sell_energy_one_kernel<<<energy_one_blocks(m.nslices), kThreads, 0, s.stream>>>(A, x, y, energy, scratch);
     else if (k == 2) launch_energy_sell<2, 1>(A, x, y, s.n, k, energy, scratch, s.stream);
     else if (k == 3) launch_energy_sell<3, 1>(A, x, y, s.n, k, energy, scratch, s.stream);
     else if (k == 4) launch_energy_sell<4, 1>(A, x, y, s.n, k, energy, scratch, s.stream);
