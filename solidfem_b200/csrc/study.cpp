@@ -465,7 +465,10 @@ static void recovery_free(sf_recovery* r);  // defined with the recovery entry p
 
 namespace {
 
-constexpr size_t kDeviceFieldNodes = 16384;           // fields of fewer nodes are spread on the host
+// Displacements of fewer nodes are spread on the host, which saves the device's temporary: 637 nodes 23
+// us a call on the host and 30 on the device, 1,701 nodes 34 and 34, 4,901 nodes 56 and 45, 18,081
+// nodes 140 and 68, 149,609 nodes 1,090 and 215.
+constexpr size_t kDeviceFieldNodes = 2048;
 
 int host_threads(const sf_study* s) {
   return s->options.threads ? (int)std::min<uint64_t>(s->options.threads, 64) : default_threads();
@@ -1245,7 +1248,7 @@ sf_status sf_builder_finish(sf_builder* b, sf_study** out) {
   copy_h2d(d, d.rhs, s->rhs.data(), (size_t)d.n * 8);
   // The conjugate gradient's f64 product runs on a SELL copy when the system has many rows.
   if (wants_sell(d.system, d.sell_min_rows))
-    if ((e = make_sell_from_device(d, d.system, s->pattern.starts.data(), s->pattern.cols.data()))) return e;
+    if ((e = make_sell_from_device(d, d.system, s->pattern.starts.data()))) return e;
   if (mg) {
     s->levels = setup_take_levels(b->setup);
     e = solver_upload_hierarchy(d, s->levels, s->options.smoother_degree);
