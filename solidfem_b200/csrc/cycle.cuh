@@ -94,17 +94,13 @@ unsigned tail_cluster_size(const HostLevel& hs, const HostLevel& hc, size_t* sme
   typedef BodyTraits<decltype(&tail_kernel<S, V>)> T;
   const void* single = T::template single_n<tail_kernel<S, V>, tail_threads<V>()>();
   const void* batched = T::template batched_n<tail_kernel<S, V>, tail_threads<V>()>();
-  // restriction row starts: the prolongator's blocks counted per coarse row
-  std::vector<uint32_t> r_starts(hc.a.rows + 1, 0);
-  for (uint32_t c : hs.p.cols) r_starts[c + 1] += 1;
-  for (size_t i = 0; i < hc.a.rows; ++i) r_starts[i + 1] += r_starts[i];
   const uint32_t nc = (uint32_t)(hc.a.rows * hc.a.rb);
   cudaFuncSetAttribute(single, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaFuncSetAttribute(batched, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   for (unsigned c : {16u, 8u}) {
     size_t bytes = 0;
     for (unsigned i = 0; i < c; ++i)
-      bytes = std::max(bytes, tail_cta_bytes(hs.a.starts, hs.p.starts, r_starts, nc, c, i, sizeof(S), sizeof(V)));
+      bytes = std::max(bytes, tail_cta_bytes(hs.a.starts, hs.p.starts, hs.t_starts, nc, c, i, sizeof(S), sizeof(V)));
     if (bytes > kTailMaxSmem) continue;
     cudaFuncSetAttribute(single, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     cudaFuncSetAttribute(batched, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);

@@ -69,8 +69,8 @@ __host__ __device__ inline size_t sell_value_offset(size_t q, int len, int chunk
 }
 
 // The SELL copy of a matrix whose values live only on the device (the assembled f64 system):
-// the layout from host starts/columns, the values permuted on the device.
-sf_status make_sell_from_device(struct DeviceSolver& s, DevBsr& m, const uint32_t* starts, const uint32_t* cols);
+// the layout from the host's row starts, columns and values permuted on the device.
+sf_status make_sell_from_device(struct DeviceSolver& s, DevBsr& m, const uint32_t* starts);
 
 // Shared memory one warp of the row-group engine may stage (two groups); the launch opts in to
 // 200 KB per block.
@@ -199,7 +199,7 @@ extern thread_local std::vector<LaunchRecord>* g_recorder;
 // Stream-ordered copies that count the bytes crossing the host-device link.
 inline void copy_h2d(const DeviceSolver& s, void* dst, const void* src, size_t bytes) {
   cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s.stream);
-  __atomic_fetch_add(&s.h2d_bytes, bytes, __ATOMIC_RELAXED);  // setup's helper thread copies too
+  __atomic_fetch_add(&s.h2d_bytes, bytes, __ATOMIC_RELAXED);
 }
 inline void copy_d2h(const DeviceSolver& s, void* dst, const void* src, size_t bytes) {
   cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s.stream);

@@ -272,8 +272,7 @@ sf_status upload_sell_layout(DeviceSolver& s, DevBsr& m, const SellLayout& L, si
 
 // The SELL copy of a matrix from its f64 values on the device, converted to S.
 template <typename S>
-sf_status make_sell_converted(DeviceSolver& s, DevBsr& m, const uint32_t* starts, const uint32_t* cols,
-                              const double* vals) {
+sf_status make_sell_converted(DeviceSolver& s, DevBsr& m, const uint32_t* starts, const double* vals) {
   const int len = (int)(m.rb * m.cb);
   SellLayout L = sell_layout(m.rows, starts, (uint32_t)sell_chunk_blocks(len, (int)sizeof(S)));
   if (sf_status e = upload_sell_layout(s, m, L, (size_t)len * sizeof(S), false)) return e;
@@ -296,9 +295,8 @@ sf_status make_split_converted(DeviceSolver& s, DevBsr& m, const uint32_t* start
   return e;
 }
 
-sf_status make_sell_from_device(DeviceSolver& s, DevBsr& m, const uint32_t* starts, const uint32_t* cols) {
-  (void)cols;
-  return make_sell_converted<double>(s, m, starts, nullptr, (const double*)m.vals);
+sf_status make_sell_from_device(DeviceSolver& s, DevBsr& m, const uint32_t* starts) {
+  return make_sell_converted<double>(s, m, starts, (const double*)m.vals);
 }
 
 namespace {
@@ -328,7 +326,7 @@ sf_status device_bsr(DeviceSolver& s, const Bsr& h, DevBsr& d, bool alias) {
   if (wants_split(d, s.uniform_lanes)) {
     if (sf_status e = make_split_converted<S>(s, d, h.starts.data(), h.dev)) return e;
   } else if (wants_sell(d, s.sell_min_rows)) {
-    if (sf_status e = make_sell_converted<S>(s, d, h.starts.data(), h.cols.data(), h.dev)) return e;
+    if (sf_status e = make_sell_converted<S>(s, d, h.starts.data(), h.dev)) return e;
   }
   return cuda_check(cudaGetLastError(), "level operator");
 }
@@ -717,18 +715,18 @@ sf_status solver_read_state(DeviceSolver& s, PcgState* out) {
 // A variant of the conjugate gradient's system product (pcg_spmv_dot_kernel and
 // sell_pcg_spmv_dot_kernel): for each of `count` vectors x_k of caller-owned device memory it
 // writes y_k = A x_k and the energy e_k = x_k . y_k. Rows are summed exactly as the system product
-// sums them; up to four vectors go through one walk of the operator, five to eight through two.
-// The reduction's scratch is not the solver's: it is
-// the file-scope array below, whose address is looked up once per device, so a call allocates no
-// memory at all.
+// sums them; up to four vectors go through one walk of the operator, five to eight through two. The
+// reduction's scratch is not the solver's: it is the file-scope array below, whose address is looked
+// up once per device, so a call allocates no memory at all.
 //
 // Scratch layout (g_energy_scratch, 262,400 bytes per device):
-//   bytes [0, 256):   one arrival ticket (unsigned) per vector. Each ticket must be zero when a
-//                     launch starts. Static device storage is zero when the module loads, and the
-//                     last block of each vector puts its ticket back to zero before it exits, so
-//                     the tickets are zero again after every completed call.
-//   bytes [256, ...): kEnergyMaxBlocks slots of partial sums per vector. No initial value is needed: every
-//                     block writes its slot before it takes its ticket.
+//   bytes [0, 256):   arrival tickets (unsigned): the first for a call on a SELL system, one per walk
+//                     on a row-group system. Each ticket must be zero when a launch starts. Static
+//                     device storage is zero when the module loads, and the last block to take a
+//                     ticket puts it back to zero before it exits, so the tickets are zero again
+//                     after every completed call.
+//   bytes [256, ...): kEnergyMaxBlocks slots of partial sums per vector. No initial value is needed:
+//                     every block writes its slots before it takes its ticket.
 // One array serves every study on a device, so two calls whose kernels can run at the same time
 // (different streams, different studies, different host threads) race on it.
 constexpr int kEnergyMaxVectors = 8;
@@ -744,11 +742,10 @@ static __device__ __align__(256) unsigned char g_energy_scratch[kEnergyScratchBy
 namespace {
 
 __device__ __forceinline__ void energy_finish(double local, unsigned char* scratch, double* energy) {
-  const uint32_t k = blockIdx.y;
-  unsigned* tickets = reinterpret_cast<unsigned*>(scratch);
-  double* partials = reinterpret_cast<double*>(scratch + kEnergyTicketBytes) + (size_t)k * kEnergyMaxBlocks;
+  unsigned* ticket = reinterpret_cast<unsigned*>(scratch);
+  double* partials = reinterpret_cast<double*>(scratch + kEnergyTicketBytes);
   double v[1] = {local}, total[1];
-  if (finish_partials<1>(v, partials, tickets + k, total) && threadIdx.x == 0) energy[k] = total[0];
+  if (finish_partials<1>(v, partials, ticket, total) && threadIdx.x == 0) energy[0] = total[0];
 }
 
 // SELL-32 system, one vector: one thread per row, rows summed as sell_kernel sums them. Bound by
@@ -908,19 +905,18 @@ __global__ void __launch_bounds__(32 * W * G) sell_energy_kernel(SellOp<double> 
   if (threadIdx.x == 0) *ticket = 0u;
 }
 
-// Row-group system: LPR lanes per row, rows summed as bsr_kernel sums them.
+// Row-group system, one vector: LPR lanes per row, rows summed as bsr_kernel sums them.
 template <int LPR>
 __global__ void __launch_bounds__(kThreads) energy_kernel(Op<double> A, const double* __restrict__ x,
-                                                           double* __restrict__ y, uint32_t n,
-                                                           double* __restrict__ energy, unsigned char* scratch) {
+                                                           double* __restrict__ y, double* __restrict__ energy,
+                                                           unsigned char* scratch) {
   extern __shared__ __align__(16) char smem[];
   char* wbase = smem + (threadIdx.x >> 5) * 2 * slot_bytes(A);
-  const size_t off = (size_t)blockIdx.y * n;
   EpiDot<LPR> epi;
-  epi.p = x + off;
-  epi.ap = y + off;
+  epi.p = x;
+  epi.ap = y;
   epi.local = 0.0;
-  run_groups<double, double, 3, 3, LPR, false>(A, x + off, wbase, epi, OpenGate{}, blockIdx.x, gridDim.x);
+  run_groups<double, double, 3, 3, LPR, false>(A, x, wbase, epi, OpenGate{}, blockIdx.x, gridDim.x);
   energy_finish(epi.local, scratch, energy);
 }
 
@@ -1060,12 +1056,11 @@ void launch_energy_sell(const SellOp<double>& A, const double* x, double* y, uin
 }
 
 template <int LPR>
-void launch_energy_lpr(const DevBsr& m, const double* x, double* y, uint32_t n, double* energy, uint64_t count,
-                       unsigned char* scratch, cudaStream_t st) {
+void launch_energy_lpr(const DevBsr& m, const double* x, double* y, double* energy, unsigned char* scratch,
+                       cudaStream_t st) {
   Op<double> A = op_of<double>(m);
   Shape sh = shape_of(A, true);
-  dim3 grid((unsigned)std::min(sh.grid, kEnergyOneBlocks), (unsigned)count);
-  energy_kernel<LPR><<<grid, sh.threads, sh.smem, st>>>(A, x, y, n, energy, scratch);
+  energy_kernel<LPR><<<std::min(sh.grid, kEnergyOneBlocks), sh.threads, sh.smem, st>>>(A, x, y, energy, scratch);
 }
 
 template <int LPR, int K>
@@ -1082,7 +1077,7 @@ template <int LPR>
 void launch_energy_rows(const DevBsr& m, const double* x, double* y, uint32_t n, double* energy, uint64_t count,
                         unsigned char* scratch, cudaStream_t st) {
   const int k = (int)count;
-  if (k == 1) launch_energy_lpr<LPR>(m, x, y, n, energy, count, scratch, st);
+  if (k == 1) launch_energy_lpr<LPR>(m, x, y, energy, scratch, st);
   else if (k == 2) launch_energy_groups<LPR, 2>(m, x, y, n, energy, k, scratch, st);
   else if (k == 3 || k == 5 || k == 6) launch_energy_groups<LPR, 3>(m, x, y, n, energy, k, scratch, st);
   else launch_energy_groups<LPR, 4>(m, x, y, n, energy, k, scratch, st);

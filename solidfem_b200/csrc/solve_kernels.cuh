@@ -38,8 +38,8 @@ const uint32_t kGroupTarget = 4096;     // value bytes a row group aims at
 const int kSmemPerBlockTarget = 72 * 1024;
 
 // ------------------------------------------------------------ programmatic dependent launch
-// Every solve kernel is launched with programmatic stream serialization. A body first requests what
-// no solve kernel ever writes (its first operator loads, D^-1), then calls pdl_wait(): it waits
+// Every solve kernel is launched with programmatic stream serialization. A body may first request
+// what no solve kernel ever writes (its first operator loads), then calls pdl_wait(): it waits
 // until the predecessor grid has completed and its writes are visible (griddepcontrol.wait), and
 // from there lets the successor's blocks start (griddepcontrol.launch_dependents) and do the same.
 // So at most the next kernel's blocks sit beside a running grid, each with its first operator loads

@@ -275,7 +275,7 @@ sf_status sf_system_create(uint64_t n, const uint64_t* row_starts, const uint32_
   std::copy(rhs, rhs + n, b.begin());
   copy_h2d(d, d.rhs, b.data(), (size_t)d.n * 8);
   if (wants_sell(d.system, d.sell_min_rows))
-    if ((e = make_sell_from_device(d, d.system, sys->starts.data(), sys->cols.data()))) return e;
+    if ((e = make_sell_from_device(d, d.system, sys->starts.data()))) return e;
   if (mg)
     if ((e = solver_upload_hierarchy(d, sys->levels, o.smoother_degree))) return e;
   if (o.device_memory_budget && d.bytes > o.device_memory_budget)
