@@ -855,9 +855,13 @@ __global__ void incidence_count_kernel(const uint32_t* __restrict__ tets10, size
   GRID_STRIDE(i, n) atomicAdd(count + tets10[i], 1u);
 }
 
-__global__ void incidence_fill_kernel(const uint32_t* __restrict__ tets10, size_t n, uint32_t* __restrict__ cursor,
-                                      uint32_t* __restrict__ inc) {
-  GRID_STRIDE(i, n) inc[atomicAdd(cursor + tets10[i], 1u)] = (uint32_t)(i / 10);
+// In any order (the sort follows), each node's list from its end.
+__global__ void incidence_fill_kernel(const uint32_t* __restrict__ tets10, size_t n, const uint32_t* __restrict__ start,
+                                      uint32_t* __restrict__ left, uint32_t* __restrict__ inc) {
+  GRID_STRIDE(i, n) {
+    const uint32_t v = tets10[i];
+    inc[start[v] + atomicSub(left + v, 1u) - 1u] = (uint32_t)(i / 10);
+  }
 }
 
 __global__ void incidence_sort_kernel(const uint32_t* __restrict__ start, uint32_t* __restrict__ inc, size_t nodes) {
@@ -941,13 +945,11 @@ __global__ void __launch_bounds__(32 * kPatternWarps) pattern_rows_kernel(
 // Each node's elements, ascending, of tets10's `nt` entries: start (nodes + 1) and inc (nt).
 sf_status enqueue_incidence(Build& b, const uint32_t* tets10, size_t nt, size_t nodes, uint32_t* start, uint32_t* inc) {
   uint32_t* count = b.alloc<uint32_t>(nodes);
-  uint32_t* cursor = b.alloc<uint32_t>(nodes);
   if (b.err) return scan_failed(b);
   cudaMemsetAsync(count, 0, nodes * 4, b.stream);
   incidence_count_kernel<<<grid_of(nt), kT, 0, b.stream>>>(tets10, nt, count);
   if (!scan(b, count, start, nodes)) return scan_failed(b);
-  cudaMemcpyAsync(cursor, start, nodes * 4, cudaMemcpyDeviceToDevice, b.stream);
-  incidence_fill_kernel<<<grid_of(nt), kT, 0, b.stream>>>(tets10, nt, cursor, inc);
+  incidence_fill_kernel<<<grid_of(nt), kT, 0, b.stream>>>(tets10, nt, start, count, inc);
   incidence_sort_kernel<<<grid_of(nodes), kT, 0, b.stream>>>(start, inc, nodes);
   return SF_OK;
 }

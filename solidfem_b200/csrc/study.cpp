@@ -1580,15 +1580,18 @@ static sf_status recovery_tables(sf_study* s) {
   DeviceSolver& d = s->solver;
   const Mesh& m = s->model.mesh;
   const size_t nn = m.nodes.size(), nv = m.vertex_count;
-  sf_status e = dev_alloc(d, (void**)&r.free, nn * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.node_offsets, (nn + 1) * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.node_incident, std::max<size_t>(1, 10 * m.tets.size()) * 4);
-  if (!e) e = dev_alloc(d, (void**)&r.midside_first, std::max<size_t>(1, nn - nv) * 4);
-  if (!e) e = copy_in(d, r.free, s->free.data(), nullptr, nn * 4, host_threads(s));
+  uint32_t* tables = nullptr;
+  sf_status e = dev_alloc(d, (void**)&tables, (nn + (nn + 1) + 10 * m.tets.size() + (nn - nv)) * 4);
+  if (e) return e;
+  r.free = tables;
+  r.node_offsets = r.free + nn;
+  r.node_incident = r.node_offsets + nn + 1;
+  r.midside_first = r.node_incident + 10 * m.tets.size();
+  e = copy_in(d, r.free, s->free.data(), nullptr, nn * 4, host_threads(s));
   if (!e) e = device_incidence(d.stream, s->asmdev.tets, m.tets.size(), nn, r.node_offsets, r.node_incident);
   if (!e) e = launch_node_incidence(s->asmdev, r, (uint32_t)nn, (uint32_t)nv, d.stream);
   if (e) {
-    for (void* p : {(void*)r.free, (void*)r.node_offsets, (void*)r.node_incident, (void*)r.midside_first}) dev_free(d, p);
+    dev_free(d, tables);
     r = RecoveryDevice();
     return e;
   }
