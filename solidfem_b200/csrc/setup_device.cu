@@ -605,26 +605,30 @@ __global__ void product_kernel(size_t entries, const uint32_t* __restrict__ entr
   }
 }
 
-// One row of a block of P^T (A P) per thread (transfer.rs:173-238): the fine rows of P's column in
-// ascending order, row r of each P block transposed times the A P block of that fine row at this
+// ROWS rows of a block of P^T (A P) per thread (transfer.rs:173-238): the fine rows of P's column in
+// ascending order, those rows of each P block transposed times the A P block of that fine row at this
 // block's column; a zero on the diagonal of a diagonal block becomes one (finish_level,
-// setup.rs:650-695). A coarse row sums tens to hundreds of fine rows and a small level has few
-// blocks, so the chain of one thread bounds it: six threads a block instead of one, each of the same
-// terms in the same order (817 blocks of about 170 fine rows: the phase 0.72 -> 0.49 ms).
-template <int N>
+// setup.rs:650-695). A coarse row sums tens to hundreds of fine rows, and where a level has few blocks
+// the chain of one thread bounds it: six threads a block then, each of the same terms in the same
+// order. Where the blocks fill the device, a whole block to a thread reads each A P block and searches
+// for it once instead of six times (kSplit below).
+template <int N, int ROWS>
 __global__ void galerkin_kernel(size_t entries, const uint32_t* __restrict__ entry_row, const uint32_t* __restrict__ c_cols,
                                 const uint32_t* __restrict__ pt_starts, const uint32_t* __restrict__ pt_rows,
                                 const uint32_t* __restrict__ pt_at, const double* __restrict__ p_vals,
                                 const uint32_t* __restrict__ ap_starts, const uint32_t* __restrict__ ap_cols,
                                 const double* __restrict__ ap_vals, double* __restrict__ c_vals) {
   constexpr int L = N * 6;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < 6 * entries; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t j = i / 6;
-    const int r = (int)(i % 6);
+  constexpr int SHARES = 6 / ROWS;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < SHARES * entries; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t j = i / SHARES;
+    const int r = (int)(i % SHARES) * ROWS;
     const uint32_t crow = entry_row[j], c = c_cols[j];
-    double acc[6];
+    double acc[ROWS][6];
 #pragma unroll
-    for (int q = 0; q < 6; ++q) acc[q] = 0.0;
+    for (int o = 0; o < ROWS; ++o)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) acc[o][q] = 0.0;
     for (uint32_t k = pt_starts[crow]; k < pt_starts[crow + 1]; ++k) {
       const uint32_t fine_row = pt_rows[k];
       const uint32_t* b = ap_cols + ap_starts[fine_row];
@@ -642,19 +646,25 @@ __global__ void galerkin_kernel(size_t entries, const uint32_t* __restrict__ ent
       const double* pb = p_vals + (size_t)pt_at[k] * L + r;
       const double* ab = ap_vals + (size_t)(lo - ap_cols) * L;
 #pragma unroll
-      for (int m = 0; m < N; ++m) {
-        double s = pb[m * 6];
+      for (int o = 0; o < ROWS; ++o)
 #pragma unroll
-        for (int q = 0; q < 6; ++q) acc[q] += s * ab[m * 6 + q];
-      }
+        for (int m = 0; m < N; ++m) {
+          double s = pb[m * 6 + o];
+#pragma unroll
+          for (int q = 0; q < 6; ++q) acc[o][q] += s * ab[m * 6 + q];
+        }
     }
     if (crow == c)
 #pragma unroll
-      for (int q = 0; q < 6; ++q)
-        if (q == r && acc[q] == 0.0) acc[q] = 1.0;
+      for (int o = 0; o < ROWS; ++o)
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+          if (q == r + o && acc[o][q] == 0.0) acc[o][q] = 1.0;
     double* out = c_vals + j * 36 + r * 6;
 #pragma unroll
-    for (int q = 0; q < 6; ++q) out[q] = acc[q];
+    for (int o = 0; o < ROWS; ++o)
+#pragma unroll
+      for (int q = 0; q < 6; ++q) out[o * 6 + q] = acc[o][q];
   }
 }
 
@@ -1337,12 +1347,20 @@ sf_status setup_galerkin(cudaStream_t st, int rb, size_t entries, const uint32_t
                          const uint32_t* pt_starts, const uint32_t* pt_rows, const uint32_t* pt_at, const double* p_vals,
                          const uint32_t* ap_starts, const uint32_t* ap_cols, const double* ap_vals, double* c_vals) {
   if (entries == 0) return SF_OK;
+  // Six threads a block up to so many blocks, one beyond. 3-row fine blocks: 10,332 blocks 360 us with
+  // six and 580 with one, 75,678 blocks 1,910 and 1,180, 307,995 blocks 1,330 and 850, 677,221 blocks
+  // 16.4 and 9.3 ms (102,624 and 412,254 blocks of plates the same either way); six threads of 32,768
+  // blocks are about what the device holds at once. 6-row fine blocks always: 11,095 blocks 810 us with
+  // six and 1,490 with one, 71,122 blocks 220 and 317, and deeper levels have no more.
+  constexpr size_t kSplit = 32768;
+  auto launch = [&](auto kernel, size_t threads) {
+    kernel<<<grid_for(threads), kT, 0, st>>>(entries, entry_row, c_cols, pt_starts, pt_rows, pt_at, p_vals, ap_starts,
+                                             ap_cols, ap_vals, c_vals);
+  };
   if (rb == 3)
-    galerkin_kernel<3><<<grid_for(6 * entries), kT, 0, st>>>(entries, entry_row, c_cols, pt_starts, pt_rows, pt_at, p_vals,
-                                                         ap_starts, ap_cols, ap_vals, c_vals);
+    entries <= kSplit ? launch(galerkin_kernel<3, 1>, 6 * entries) : launch(galerkin_kernel<3, 6>, entries);
   else
-    galerkin_kernel<6><<<grid_for(6 * entries), kT, 0, st>>>(entries, entry_row, c_cols, pt_starts, pt_rows, pt_at, p_vals,
-                                                         ap_starts, ap_cols, ap_vals, c_vals);
+    launch(galerkin_kernel<6, 1>, 6 * entries);
   return cuda_check(cudaGetLastError(), "galerkin");
 }
 
