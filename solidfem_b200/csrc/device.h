@@ -259,11 +259,13 @@ sf_status setup_strength(cudaStream_t st, uint32_t rows, const uint32_t* starts,
 sf_status setup_union_rows(cudaStream_t st, uint32_t rows, uint32_t width, const uint32_t* outer_starts,
                            const uint32_t* outer_idx, bool self, const uint32_t* inner_starts,
                            const uint32_t* inner_cols, const uint32_t* out_starts, uint32_t* out);
-// The 3x3 blocks of a scalar CSR matrix of n rows (columns ascending) over `rows` = ceil(n / 3) block
-// rows, the padding rows' diagonal included: out_starts null counts each block row's blocks into
-// out; else the block columns go to out[out_starts[row] ..] and the entries into vals (zeros before).
-sf_status setup_padded_blocks(cudaStream_t st, uint64_t n, uint32_t rows, const uint64_t* rs, const uint32_t* cols,
-                              const double* scalars, const uint32_t* out_starts, uint32_t* out, double* vals);
+// The 3x3 blocks of a scalar CSR matrix of n rows (columns ascending) in the block rows [first, end) of
+// ceil(n / 3), the padding rows' diagonal included; cols and scalars hold the entries from `entry` on.
+// out_starts null counts each block row's blocks into out; else the block columns go to
+// out[out_starts[row] ..] and the entries into vals (zeros before).
+sf_status setup_padded_blocks(cudaStream_t st, uint64_t n, uint32_t first, uint32_t end, uint64_t entry,
+                              const uint64_t* rs, const uint32_t* cols, const double* scalars,
+                              const uint32_t* out_starts, uint32_t* out, double* vals);
 // Listed blocks of len values out of / back into a block array; out[idx[i]] = vals[i].
 sf_status setup_gather_blocks(cudaStream_t st, size_t count, int len, const uint32_t* idx, const double* in,
                               double* out);

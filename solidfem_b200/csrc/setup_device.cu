@@ -1003,19 +1003,20 @@ __device__ __forceinline__ uint32_t lanes_below(uint32_t block, uint32_t key) {
 // strictly ascending, so a block has three entries of a row at most and every step takes 29 or more
 // of some row. A thread per block row read a dense row as one chain of loads: 91,125 unknowns with
 // one full row and column were created in 48 ms.
-__global__ void padded_blocks_kernel(uint64_t n, uint32_t rows, const uint64_t* __restrict__ rs,
-                                     const uint32_t* __restrict__ cols, const double* __restrict__ scalars,
+// Block rows [first_row, end_row); cols and scalars hold the entries from `entry` on.
+__global__ void padded_blocks_kernel(uint64_t n, uint32_t first_row, uint32_t end_row, uint64_t entry,
+                                     const uint64_t* __restrict__ rs, const uint32_t* __restrict__ cols, const double* __restrict__ scalars,
                                      const uint32_t* __restrict__ out_starts, uint32_t* __restrict__ out,
                                      double* __restrict__ vals) {
   constexpr uint32_t kNone = 0xffffffffu;  // past a row's end
-  const uint32_t lane = threadIdx.x & 31, b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (b >= rows) return;
-  uint64_t at[3], end[3];
+  const uint32_t lane = threadIdx.x & 31, b = first_row + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (b >= end_row) return;
+  uint64_t at[3], end[3];  // within cols and scalars
 #pragma unroll
   for (int p = 0; p < 3; ++p) {
     const uint64_t r = 3 * (uint64_t)b + p;
-    at[p] = r < n ? rs[r] : 0;
-    end[p] = r < n ? rs[r + 1] : 0;
+    at[p] = r < n ? rs[r] - entry : 0;
+    end[p] = r < n ? rs[r + 1] - entry : 0;
   }
   bool own = 3 * (uint64_t)b + 3 > n;  // the padding's diagonal block is still to come
   const size_t base = out_starts ? out_starts[b] : 0;
@@ -1099,10 +1100,12 @@ __global__ void set_values_kernel(size_t count, const uint32_t* __restrict__ idx
 
 }  // namespace
 
-sf_status setup_padded_blocks(cudaStream_t st, uint64_t n, uint32_t rows, const uint64_t* rs, const uint32_t* cols,
-                              const double* scalars, const uint32_t* out_starts, uint32_t* out, double* vals) {
-  if (rows == 0) return SF_OK;
-  padded_blocks_kernel<<<(rows + 3) / 4, 128, 0, st>>>(n, rows, rs, cols, scalars, out_starts, out, vals);
+sf_status setup_padded_blocks(cudaStream_t st, uint64_t n, uint32_t first, uint32_t end, uint64_t entry,
+                              const uint64_t* rs, const uint32_t* cols, const double* scalars,
+                              const uint32_t* out_starts, uint32_t* out, double* vals) {
+  if (end <= first) return SF_OK;
+  padded_blocks_kernel<<<(end - first + 3) / 4, 128, 0, st>>>(n, first, end, entry, rs, cols, scalars, out_starts, out,
+                                                              vals);
   return cuda_check(cudaGetLastError(), "padded blocks");
 }
 

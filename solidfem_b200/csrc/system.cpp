@@ -110,35 +110,54 @@ sf_status from_nodal(uint64_t n, const uint64_t* rs, const uint32_t* cols, const
 
 // Any scalar matrix over ceil(n / 3) block rows, on the device from its scalar rows: the blocks its
 // entries touch (and the last diagonal block when padding rows are added), zeros where it has no
-// entry, identity on the padding's diagonal. `starts` gets the block rows' starts.
+// entry, identity on the padding's diagonal. `starts` gets the block rows' starts. The scalar rows
+// cross in parts of kPartEntries (a block row at least), so that they take no more of the device than
+// the solve's own arrays will.
+constexpr uint64_t kPartEntries = (uint64_t)1 << 22;
+
 sf_status padded_blocks(DeviceSolver& d, uint64_t n, const uint64_t* rs, const uint32_t* cols, const double* vals,
                         vector<uint32_t>& starts) {
-  const size_t rows = d.system.rows, entries = rs[n];
+  const uint32_t rows = d.system.rows;
+  auto entry = [&](uint32_t block_row) { return rs[std::min<uint64_t>(3 * (uint64_t)block_row, n)]; };
+  vector<uint32_t> cuts(1, 0);
+  uint64_t largest = 1;
+  while (cuts.back() < rows) {
+    uint32_t e = cuts.back() + 1;
+    while (e < rows && entry(e + 1) - entry(cuts.back()) <= kPartEntries) ++e;
+    largest = std::max(largest, entry(e) - entry(cuts.back()));
+    cuts.push_back(e);
+  }
   uint64_t* d_rs = nullptr;
   uint32_t* d_cols = nullptr;
   double* d_vals = nullptr;
   sf_status e = dev_alloc(d, (void**)&d_rs, (n + 1) * 8);
-  if (!e) e = dev_alloc(d, (void**)&d_cols, std::max<size_t>(1, entries) * 4);
-  if (!e) e = dev_alloc(d, (void**)&d_vals, std::max<size_t>(1, entries) * 8);
+  if (!e) e = dev_alloc(d, (void**)&d_cols, largest * 4);
   if (e) return e;
   copy_h2d(d, d_rs, rs, (n + 1) * 8);
-  if (entries) {
-    copy_h2d(d, d_cols, cols, entries * 4);
-    copy_h2d(d, d_vals, vals, entries * 8);
+  const bool whole = cuts.size() == 2;  // the columns of the first pass serve the second
+  for (size_t i = 0; i + 1 < cuts.size() && !e; ++i) {
+    const uint64_t lo = entry(cuts[i]), hi = entry(cuts[i + 1]);
+    if (hi > lo) copy_h2d(d, d_cols, cols + lo, (hi - lo) * 4);
+    e = setup_padded_blocks(d.stream, n, cuts[i], cuts[i + 1], lo, d_rs, d_cols, nullptr, nullptr, d.system.starts, nullptr);
   }
-  e = setup_padded_blocks(d.stream, n, (uint32_t)rows, d_rs, d_cols, d_vals, nullptr, d.system.starts, nullptr);
   starts.assign(rows + 1, 0);
-  if (!e) copy_d2h(d, starts.data() + 1, d.system.starts, rows * 4);
+  if (!e) copy_d2h(d, starts.data() + 1, d.system.starts, (size_t)rows * 4);
   if (!e) e = cuda_check(cudaStreamSynchronize(d.stream), "system blocks");
   if (e) return e;
   for (size_t r = 0; r < rows; ++r) starts[r + 1] += starts[r];
   const size_t blocks = d.system.blocks = starts[rows];
+  if (!e) e = dev_alloc(d, (void**)&d_vals, largest * 8);
   if (!e) e = dev_alloc(d, (void**)&d.system.cols, std::max<size_t>(1, blocks) * 4);
   if (!e) e = dev_alloc(d, &d.system.vals, std::max<size_t>(1, blocks) * 72);  // zeros
   if (e) return e;
-  copy_h2d(d, d.system.starts, starts.data(), (rows + 1) * 4);
-  e = setup_padded_blocks(d.stream, n, (uint32_t)rows, d_rs, d_cols, d_vals, d.system.starts, d.system.cols,
-                          (double*)d.system.vals);
+  copy_h2d(d, d.system.starts, starts.data(), ((size_t)rows + 1) * 4);
+  for (size_t i = 0; i + 1 < cuts.size() && !e; ++i) {
+    const uint64_t lo = entry(cuts[i]), hi = entry(cuts[i + 1]);
+    if (hi > lo && !whole) copy_h2d(d, d_cols, cols + lo, (hi - lo) * 4);
+    if (hi > lo) copy_h2d(d, d_vals, vals + lo, (hi - lo) * 8);
+    e = setup_padded_blocks(d.stream, n, cuts[i], cuts[i + 1], lo, d_rs, d_cols, d_vals, d.system.starts, d.system.cols,
+                            (double*)d.system.vals);
+  }
   for (void* p : {(void*)d_rs, (void*)d_cols, (void*)d_vals}) dev_free(d, p);
   return e;
 }
