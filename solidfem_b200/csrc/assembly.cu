@@ -755,9 +755,9 @@ __global__ void scatter_displacements_kernel(const double* __restrict__ x, const
 __global__ void node_incidence_kernel(const uint32_t* __restrict__ tets, uint32_t nodes, uint32_t vertices,
                                       const uint32_t* __restrict__ inc_start, uint32_t* __restrict__ incident,
                                       uint32_t* __restrict__ midside_first) {
-  const uint32_t n = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // a warp per node
   if (n >= nodes) return;
-  for (uint32_t k = inc_start[n]; k < inc_start[n + 1]; ++k) {
+  for (uint32_t k = inc_start[n] + (threadIdx.x & 31); k < inc_start[n + 1]; k += 32) {
     const uint32_t e = incident[k];
     uint32_t a = 0;
     while (a < 9 && tets[(size_t)e * 10 + a] != n) ++a;
@@ -796,7 +796,7 @@ sf_status launch_scatter_displacements(const double* x, const uint32_t* free, si
 
 sf_status launch_node_incidence(const AssemblyDevice& a, RecoveryDevice& r, uint32_t node_count, uint32_t vertex_count,
                                 cudaStream_t stream) {
-  node_incidence_kernel<<<(node_count + 127) / 128, 128, 0, stream>>>(a.tets, node_count, vertex_count, r.node_offsets,
+  node_incidence_kernel<<<(node_count + 3) / 4, 128, 0, stream>>>(a.tets, node_count, vertex_count, r.node_offsets,
                                                                       r.node_incident, r.midside_first);
   return cuda_check(cudaGetLastError(), "recovery incidence");
 }
